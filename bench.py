@@ -698,8 +698,8 @@ class MeshWorkload:
     (3,968 triangles) into a 128^3 signed-distance grid (pf_bake_sdf);
     `voxelize` fills a 48 x 24 torus (2,304 triangles) with particles of
     radius 2.5 mm (pf_voxelize_mesh, about 1.9 M grid points). The unit is
-    grid-point x triangle tests per second (the brute force both the
-    reference and this build run)."""
+    grid-point x triangle pairs per second: the pairs of the reference's
+    brute force (the bake leaves out those that cannot matter)."""
 
     unit = "point-triangle tests/s"
 
