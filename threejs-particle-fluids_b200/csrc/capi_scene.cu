@@ -801,6 +801,7 @@ pf_status pf_loop_build(pf_scene* s, const pf_loop_desc* d) {
     s->spec.built = false;
     return st;
   }
+  w->graph_later();
   s->world = std::move(w);
   return PF_OK;
 }

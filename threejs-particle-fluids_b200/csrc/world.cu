@@ -2982,12 +2982,12 @@ pf_status World::step(double dt) {
       if (any_grid_) p ^= 1;
     }
   };
-  if (use_graph_) {
-    // Both start parities are captured on the first step, so later steps
-    // only launch (no capture runs while a host thread builds another world).
-    // After the grid windows grew, the captured steps are captured again
-    // and, where the launches keep their shape, updated in place (cheaper
-    // than a new instantiation).
+  // Both start parities are captured on the first step (a plain scene's on
+  // its kGraphAfter-th), so later steps only launch (no capture runs while a
+  // host thread builds another world). After the grid windows grew, the
+  // captured steps are captured again and, where the launches keep their
+  // shape, updated in place (cheaper than a new instantiation).
+  auto capture = [&]() -> pf_status {
     const uint32_t parities[2] = {parity_, parity_ ^ flips};
     for (uint32_t i = 0; i < (flips ? 2u : 1u); ++i) {
       const uint32_t p = parities[i];
@@ -3019,6 +3019,20 @@ pf_status World::step(double dt) {
                      std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_cap).count());
     }
     graphs_stale_ = false;
+    return PF_OK;
+  };
+  bool graph = use_graph_;
+  if (graph) {
+    PF_TRY(capture());
+  } else if (lazy_graph_ && steps_done_ >= kGraphAfter) {
+    // a plain scene whose capture fails (no memory for it) steps on without
+    graph = lazy_graph_ = capture() == PF_OK;
+    if (!graph) {
+      cudaGetLastError();
+      drop_graphs();
+    }
+  }
+  if (graph) {
     PF_CUDA(cudaGraphLaunch(graph_[parity_], stream_));
   } else {
     body(parity_);
