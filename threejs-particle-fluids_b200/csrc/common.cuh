@@ -58,6 +58,67 @@ enum DeviceError : uint32_t {
 // tile ids taken in launch order, so this only triggers on a bug).
 constexpr uint32_t kLookbackSpinLimit = 1u << 24;
 
+// ------------------------------------------------- linked launches ----
+// A stage of a step or a sort is a few microseconds of kernel, and a plain
+// launch adds a microsecond or two of starting it after the kernel before
+// has completed. Kernels launched one after the other on a stream inside a
+// LinkedLaunches scope are therefore linked (programmatic dependent launch):
+// the next kernel's blocks are placed once the blocks of the one before have
+// exited, and wait in pdl_begin(), their first statement, until its writes
+// are visible. Nothing of a kernel runs before its pdl_begin(), so the order
+// of the work is that of plain launches. No kernel signals its dependents
+// earlier: blocks placed beside a running kernel crowded on the SMs that it
+// left first, which made the soft-body passes 7 % slower (24 mixed scenes:
+// 2.67 ms a step plain, 2.87 signalled at the start, 2.64 at the exit).
+// Plain and linked: a sort of 20,011 particles 57 and 40 us, of 1,000,003
+// 103 and 72, a 256 x 256 cloth's step (190 launches) 0.86 and 0.81 ms, a
+// 30,000-particle fluid's with surface effects (307) 2.31 and 2.24.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The calling thread's state: linking is on inside a scope, and the last
+// operation issued there was a kernel on `last`.
+struct LinkState {
+  bool on = false, linked = false;
+  cudaStream_t last = nullptr;
+};
+inline thread_local LinkState t_link;
+
+// Links the launches of its lifetime; what came before is waited for in full.
+class LinkedLaunches {
+ public:
+  LinkedLaunches() : was_(t_link) { t_link = LinkState{true, false, nullptr}; }
+  ~LinkedLaunches() { t_link = was_; }
+  LinkedLaunches(const LinkedLaunches&) = delete;
+  LinkedLaunches& operator=(const LinkedLaunches&) = delete;
+
+ private:
+  LinkState was_;
+};
+// To be called after any operation other than launch_kernel (a copy, a
+// memset, a wait for another stream's event): the next kernel is launched
+// plainly, after all of the stream's work before it.
+inline void break_link() { t_link.linked = false; }
+
+// kernel<<<grid, block, smem, st>>>(args...), linked where the operation
+// before it on this thread was a kernel on the same stream. Every kernel
+// launched through it starts with pdl_begin().
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = t_link.on && t_link.linked && t_link.last == st ? 1 : 0;
+  t_link.linked = true;
+  t_link.last = st;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 __host__ __device__ inline uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 }  // namespace pf

@@ -120,8 +120,8 @@ __device__ __forceinline__ void store_status(uint64_t* p, uint64_t v) {
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t* __restrict__ zero_out,
-       uint64_t n, uint64_t* __restrict__ status, uint32_t* __restrict__ counters, uint32_t vec) {
+k_scan(const uint32_t* in, uint32_t* out, uint64_t n, uint64_t* status, uint32_t* counters, uint32_t vec) {
+  pdl_begin();
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[kScanThreads / 32];
   __shared__ uint32_t s_prefix;
@@ -217,18 +217,10 @@ k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t* __
 #pragma unroll
     for (int q = 0; q < (int)kScanItems / 4; ++q)
       dst[q] = make_uint4(prefix + v[4 * q], prefix + v[4 * q + 1], prefix + v[4 * q + 2], prefix + v[4 * q + 3]);
-    if (zero_out) {
-      uint4* z = reinterpret_cast<uint4*>(zero_out + base);
-#pragma unroll
-      for (int q = 0; q < (int)kScanItems / 4; ++q) z[q] = make_uint4(0, 0, 0, 0);
-    }
   } else {
 #pragma unroll
     for (int k = 0; k < (int)kScanItems; ++k)
-      if (base + k < n) {
-        out[base + k] = prefix + v[k];
-        if (zero_out) zero_out[base + k] = 0;
-      }
+      if (base + k < n) out[base + k] = prefix + v[k];
   }
 }
 
@@ -236,21 +228,24 @@ k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t* __
 // -------------------------------------------------------- keys + digits ----
 // Keys of every element with the radix digit counts of every pass, in a
 // grid-stride loop: each block keeps its digit histograms in shared memory
-// and adds them to the global counts once.
+// and adds them to the global counts once. The cell counts are zeroed here
+// (the last pass adds to them).
 __global__ void __launch_bounds__(kHistThreads)
-k_keys_digits(const float4* __restrict__ pos, uint32_t n, KeyFn kf, DigitHist h, uint32_t* __restrict__ keys,
-              uint32_t* __restrict__ overflow) {
+k_keys_digits(const float4* pos, uint32_t n, KeyFn kf, DigitHist h, uint32_t* keys, uint32_t* overflow,
+              uint32_t* count, uint64_t cells) {
+  pdl_begin();
   extern __shared__ uint32_t sh[];
   digit_hist_zero(sh, h);
   __syncthreads();
   uint32_t over_any = 0;
   const uint32_t stride = gridDim.x * blockDim.x;
+  zero_counts(count, cells);
   // kKeysUnroll positions in flight per thread before their keys
   for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kKeysUnroll * stride) {
     float4 p[kKeysUnroll];
 #pragma unroll
     for (uint32_t q = 0; q < kKeysUnroll; ++q)
-      if (i0 + q * stride < n) p[q] = __ldg(pos + i0 + q * stride);
+      if (i0 + q * stride < n) p[q] = pos[i0 + q * stride];
 #pragma unroll
     for (uint32_t q = 0; q < kKeysUnroll; ++q) {
       const uint32_t i = i0 + q * stride;
@@ -270,6 +265,7 @@ k_keys_digits(const float4* __restrict__ pos, uint32_t n, KeyFn kf, DigitHist h,
 // Each pass's digit counts -> each digit's first output position (one block
 // of 1024 threads per pass, two digits per thread).
 __global__ void __launch_bounds__(1024) k_digit_first(uint32_t* __restrict__ dc, uint32_t digits) {
+  pdl_begin();
   __shared__ uint32_t s_warp[32];
   uint32_t* c = dc + blockIdx.x * kRadixMaxDigits;
   const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
@@ -306,8 +302,8 @@ static_assert(kCountItems % 4 == 0, "tile count loads");
 // Digit counts of tile blockIdx.x: row tile of `tcount` (digits entries).
 // `vec`: kin is 16-byte aligned (whole tiles load four keys at a time).
 __global__ void __launch_bounds__(kCountThreads)
-k_tile_counts(const uint32_t* __restrict__ kin, uint32_t n, uint32_t shift, uint32_t digits,
-              uint32_t* __restrict__ tcount, uint32_t vec) {
+k_tile_counts(const uint32_t* kin, uint32_t n, uint32_t shift, uint32_t digits, uint32_t* tcount, uint32_t vec) {
+  pdl_begin();
   __shared__ uint32_t h[kRadixMaxDigits];
   for (uint32_t d = threadIdx.x; d < digits; d += kCountThreads) h[d] = 0u;
   __syncthreads();
@@ -317,7 +313,7 @@ k_tile_counts(const uint32_t* __restrict__ kin, uint32_t n, uint32_t shift, uint
     const uint4* src = reinterpret_cast<const uint4*>(kin + base);
     uint4 v[kCountItems / 4];
 #pragma unroll
-    for (uint32_t q = 0; q < kCountItems / 4; ++q) v[q] = __ldg(src + threadIdx.x + q * kCountThreads);
+    for (uint32_t q = 0; q < kCountItems / 4; ++q) v[q] = src[threadIdx.x + q * kCountThreads];
 #pragma unroll
     for (uint32_t q = 0; q < kCountItems / 4; ++q) {
       atomicAdd(h + ((v[q].x >> shift) & mask), 1u);
@@ -329,7 +325,7 @@ k_tile_counts(const uint32_t* __restrict__ kin, uint32_t n, uint32_t shift, uint
 #pragma unroll 4
     for (uint32_t i = threadIdx.x; i < kRadixTile; i += kCountThreads) {
       const size_t e = base + i;
-      if (e < n) atomicAdd(h + ((__ldg(kin + e) >> shift) & mask), 1u);
+      if (e < n) atomicAdd(h + ((kin[e] >> shift) & mask), 1u);
     }
   }
   __syncthreads();
@@ -342,8 +338,8 @@ k_tile_counts(const uint32_t* __restrict__ kin, uint32_t n, uint32_t shift, uint
 // `first` (a pass of one chunk), csum gets the digit's first output position
 // instead, so no scan over the chunks is needed.
 __global__ void __launch_bounds__(256)
-k_tile_scan_chunk(uint32_t* __restrict__ tcount, uint32_t tiles, uint32_t digits, uint32_t* __restrict__ csum,
-                  const uint32_t* __restrict__ first) {
+k_tile_scan_chunk(uint32_t* tcount, uint32_t tiles, uint32_t digits, uint32_t* csum, const uint32_t* first) {
+  pdl_begin();
   const uint32_t d = blockIdx.y * blockDim.x + threadIdx.x;
   if (d >= digits) return;
   const uint32_t t0 = blockIdx.x * kScanChunk, t1 = min(t0 + kScanChunk, tiles);
@@ -363,7 +359,8 @@ k_tile_scan_chunk(uint32_t* __restrict__ tcount, uint32_t tiles, uint32_t digits
 // chunk's first output position (the digit's first position plus the counts
 // of the chunks before), in place.
 __global__ void __launch_bounds__(256)
-k_tile_scan_chunks(uint32_t* __restrict__ csum, uint32_t chunks, uint32_t digits, const uint32_t* __restrict__ first) {
+k_tile_scan_chunks(uint32_t* csum, uint32_t chunks, uint32_t digits, const uint32_t* first) {
+  pdl_begin();
   const uint32_t d = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const uint32_t lane = lane_id();
   if (d >= digits) return;  // whole warps
@@ -445,10 +442,9 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, uint32_t bits, uint3
 // entries to count[key] (the cell counts of the sort).
 template <bool kFirst, bool kLast, bool kBallot, uint32_t kW>
 __global__ void __launch_bounds__(kOsThreads, 2)
-k_radix_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t n,
-                uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t shift, uint32_t digits,
-                const uint32_t* __restrict__ tcount, const uint32_t* __restrict__ csum,
-                uint32_t* __restrict__ count, uint32_t vec) {
+k_radix_scatter(const uint32_t* kin, const uint32_t* vin, uint32_t n, uint32_t* kout, uint32_t* vout, uint32_t shift,
+                uint32_t digits, const uint32_t* tcount, const uint32_t* csum, uint32_t* count, uint32_t vec) {
+  pdl_begin();
   extern __shared__ __align__(16) uint32_t sm[];
   uint32_t* in_k = sm;                                                  // [2][kRadixTile]
   uint32_t* in_v = sm + 2 * kRadixTile;                                 // [2][kRadixTile], not with kFirst
@@ -480,7 +476,7 @@ k_radix_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ v
     {
       const uint32_t* trow = tcount + (size_t)tile * digits;
       const uint32_t* crow = csum + (size_t)(tile / kScanChunk) * digits;
-      for (uint32_t d = tid; d < digits; d += kOsThreads) gstart[d] = __ldg(trow + d) + __ldg(crow + d);
+      for (uint32_t d = tid; d < digits; d += kOsThreads) gstart[d] = trow[d] + crow[d];
     }
     uint32_t* wrow = reinterpret_cast<uint32_t*>(whist + warp * digits);  // digits is even
     for (uint32_t w = lane; w < digits / 2; w += 32) wrow[w] = 0u;
@@ -619,18 +615,19 @@ k_radix_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ v
 
 // A plan of no passes (one cell): the identity permutation.
 __global__ void __launch_bounds__(256) k_identity(uint32_t* __restrict__ perm, uint32_t n) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) perm[i] = i;
 }
 
 // Cell counts from the sorted keys: one atomic per run of equal keys in a
 // warp (a run's first lane in the warp adds the run's length there).
-__global__ void __launch_bounds__(256) k_run_counts(const uint32_t* __restrict__ sk, uint32_t n,
-                                                    uint32_t* __restrict__ count) {
+__global__ void __launch_bounds__(256) k_run_counts(const uint32_t* sk, uint32_t n, uint32_t* count) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = lane_id();
   const bool valid = i < n;
-  const uint32_t key = valid ? __ldg(sk + i) : 0xffffffffu;
+  const uint32_t key = valid ? sk[i] : 0xffffffffu;
   const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
   const bool starts = valid && (lane == 0 || key != prev);
   const uint32_t heads = __ballot_sync(0xffffffffu, starts);
@@ -722,8 +719,9 @@ RadixPlan radix_plan(uint64_t cells) {
 
 uint32_t scan_tiles(uint64_t n) { return (uint32_t)((n + kScanTile - 1) / kScanTile); }
 
-uint32_t keys_grid(uint32_t n, uint32_t threads) {
-  return std::max<uint32_t>(1, std::min<uint32_t>(div_up(std::max<uint32_t>(n, 1), threads), (uint32_t)sm_count() * 8));
+uint32_t keys_grid(uint32_t n, uint64_t cells, uint32_t threads) {
+  const uint64_t items = std::max<uint64_t>(std::max<uint64_t>(n, cells / 4), 1);
+  return (uint32_t)std::min<uint64_t>((items + threads - 1) / threads, (uint64_t)sm_count() * 8);
 }
 
 namespace {
@@ -734,11 +732,12 @@ uint32_t radix_tiles(uint32_t n) { return std::max<uint32_t>(1, div_up(n, kRadix
 size_t sort_scratch_bytes(uint32_t n, uint64_t C) {
   size_t b = 0;
   b += 5 * align256(4ull * n);                                          // keys, ka, va, kb, vb
-  b += align256(4ull * kRadixMaxPasses * kRadixMaxDigits);             // digit counts
   b += align256(4ull * radix_tiles(n) * kRadixMaxDigits);                 // tile digit counts
   b += align256(4ull * div_up(radix_tiles(n), kScanChunk) * kRadixMaxDigits);  // chunk bases
-  b += align256(8ull * scan_tiles(std::max<uint64_t>(C, 1)));           // scan tile status
+  // what a sort finds zeroed (sort_state_zero): one range
+  b += align256(4ull * kRadixMaxPasses * kRadixMaxDigits);             // digit counts
   b += align256(4ull * kNumCounters);                                   // counters
+  b += align256(8ull * scan_tiles(std::max<uint64_t>(C, 1)));           // scan tile status
   return b;
 }
 
@@ -754,43 +753,45 @@ void sort_scratch_carve(void* base, uint32_t n, uint64_t C, SortScratch* s) {
   s->va = reinterpret_cast<uint32_t*>(take(4ull * n));
   s->kb = reinterpret_cast<uint32_t*>(take(4ull * n));
   s->vb = reinterpret_cast<uint32_t*>(take(4ull * n));
-  s->digit_count = reinterpret_cast<uint32_t*>(take(4ull * kRadixMaxPasses * kRadixMaxDigits));
   s->tiles_cap = radix_tiles(n);
   s->tcount = reinterpret_cast<uint32_t*>(take(4ull * s->tiles_cap * kRadixMaxDigits));
   s->csum = reinterpret_cast<uint32_t*>(take(4ull * div_up(s->tiles_cap, kScanChunk) * kRadixMaxDigits));
+  s->digit_count = reinterpret_cast<uint32_t*>(take(4ull * kRadixMaxPasses * kRadixMaxDigits));
+  s->counters = reinterpret_cast<uint32_t*>(take(4ull * kNumCounters));
   s->scan_tiles_cap = scan_tiles(std::max<uint64_t>(C, 1));
   s->scan_status = reinterpret_cast<uint64_t*>(take(8ull * s->scan_tiles_cap));
-  s->counters = reinterpret_cast<uint32_t*>(take(4ull * kNumCounters));
   s->n_cap = n;
   s->c_cap = (uint32_t)C;
 }
 
 cudaError_t sort_scratch_zero(const SortScratch& s, cudaStream_t st) {
-  // the digit counts, tile counts, chunk bases, scan status and counters
+  // the tile counts, chunk bases, digit counts, counters and scan status
+  const char* a = reinterpret_cast<const char*>(s.tcount);
+  const char* b = reinterpret_cast<const char*>(s.scan_status) + 8ull * s.scan_tiles_cap;
+  return cudaMemsetAsync(const_cast<char*>(a), 0, (size_t)(b - a), st);
+}
+
+cudaError_t sort_state_zero(const SortScratch& s, uint64_t C, cudaStream_t st) {
   const char* a = reinterpret_cast<const char*>(s.digit_count);
-  const char* b = reinterpret_cast<const char*>(s.counters) + 4ull * kNumCounters;
+  const char* b = reinterpret_cast<const char*>(s.scan_status) + 8ull * scan_tiles(C);
+  break_link();
   return cudaMemsetAsync(const_cast<char*>(a), 0, (size_t)(b - a), st);
 }
 
 void launch_keys_digits(const float4* pos, uint32_t n, const KeyFn& kf, const RadixPlan& plan, uint32_t* keys,
-                        uint32_t* overflow, const SortScratch& s, cudaStream_t st) {
-  if (n == 0) return;
+                        uint32_t* overflow, uint32_t* count, uint64_t C, const SortScratch& s, cudaStream_t st) {
   const DigitHist h = digit_hist(plan, s);
-  k_keys_digits<<<keys_grid(n, kHistThreads), kHistThreads, 4ull * plan.passes * plan.digits, st>>>(pos, n, kf, h, keys,
-                                                                                                   overflow);
+  launch_kernel(k_keys_digits, keys_grid(n, C, kHistThreads), kHistThreads, 4ull * plan.passes * plan.digits, st, pos, n, kf, h, keys,
+                overflow, count, C);
 }
 
-cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t* zero_out, uint64_t n,
-                                  uint64_t* tile_status, uint32_t* counters, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const uint32_t tiles = scan_tiles(n);
-  if (cudaError_t e = cudaMemsetAsync(tile_status, 0, 8ull * tiles, st); e != cudaSuccess) return e;
-  if (cudaError_t e = cudaMemsetAsync(counters + kCounterTicket, 0, 4, st); e != cudaSuccess) return e;
-  const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) |
-                     reinterpret_cast<uintptr_t>(zero_out)) & 15u) == 0;
-  k_scan<<<tiles, kScanThreads, 0, st>>>(in, out, zero_out, n, tile_status, counters, vec ? 1u : 0u);
-  return cudaGetLastError();
+namespace {
+// Cell counts -> cell starts (its tile status and ticket zeroed before).
+cudaError_t launch_start_scan(const uint32_t* in, uint32_t* out, uint64_t n, const SortScratch& s, cudaStream_t st) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  return launch_kernel(k_scan, scan_tiles(n), kScanThreads, 0, st, in, out, n, s.scan_status, s.counters, vec ? 1u : 0u);
 }
+}  // namespace
 
 namespace {
 // Per device: shared memory per SM, for the blocks per SM of the persistent
@@ -819,8 +820,7 @@ cudaError_t launch_scatter_as(const uint32_t* kin, const uint32_t* vin, uint32_t
   const uint32_t grid = std::min<uint32_t>(radix_tiles(n), blocks * (uint32_t)sm_count());
   const bool vec = (reinterpret_cast<uintptr_t>(kin) & 15u) == 0 &&
                    (kFirst || (reinterpret_cast<uintptr_t>(vin) & 15u) == 0);
-  k_radix_scatter<kFirst, kLast, kBallot, kW><<<grid, kOsThreads, smem, st>>>(
-      kin, vin, n, kout, vout, shift, plan.digits, s.tcount, s.csum, count, vec ? 1u : 0u);
+  launch_kernel(k_radix_scatter<kFirst, kLast, kBallot, kW>, grid, kOsThreads, smem, st, kin, vin, n, kout, vout, shift, plan.digits, s.tcount, s.csum, count, vec ? 1u : 0u);
   return cudaGetLastError();
 }
 
@@ -872,15 +872,14 @@ uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n) {
 cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan, uint32_t* count,
                              uint32_t* start, uint32_t* perm, const SortScratch& s, cudaStream_t st) {
   if (C == 0) return cudaSuccess;
-  if (cudaError_t e = cudaMemsetAsync(count, 0, 4ull * C, st); e != cudaSuccess) return e;
   if (n > 0) {
     const uint32_t tiles = radix_tiles(n);
     if (plan.passes == 0) {
-      k_identity<<<div_up(n, 256), 256, 0, st>>>(perm, n);
-      k_run_counts<<<div_up(n, 256), 256, 0, st>>>(keys, n, count);
+      launch_kernel(k_identity, div_up(n, 256), 256, 0, st, perm, n);
+      launch_kernel(k_run_counts, div_up(n, 256), 256, 0, st, keys, n, count);
     } else {
       if (cudaError_t e = radix_prepare(); e != cudaSuccess) return e;
-      k_digit_first<<<plan.passes, 1024, 0, st>>>(s.digit_count, plan.digits);
+      launch_kernel(k_digit_first, plan.passes, 1024, 0, st, s.digit_count, plan.digits);
       const uint32_t chunks = div_up(tiles, kScanChunk);
       const bool kvec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
       const uint32_t* kin = keys;
@@ -892,13 +891,12 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
         uint32_t* kout = last ? nullptr : ((p & 1u) ? s.kb : s.ka);
         uint32_t* vout = last ? perm : ((p & 1u) ? s.vb : s.va);
         const uint32_t shift = p * plan.width;
-        k_tile_counts<<<tiles, kCountThreads, 0, st>>>(kin, n, shift, plan.digits, s.tcount,
+        launch_kernel(k_tile_counts, tiles, kCountThreads, 0, st, kin, n, shift, plan.digits, s.tcount,
                                                        (first ? kvec : true) ? 1u : 0u);
         const uint32_t* first_pos = s.digit_count + p * kRadixMaxDigits;
-        k_tile_scan_chunk<<<dim3(chunks, div_up(plan.digits, 256)), 256, 0, st>>>(
-            s.tcount, tiles, plan.digits, s.csum, chunks == 1 ? first_pos : nullptr);
+        launch_kernel(k_tile_scan_chunk, dim3(chunks, div_up(plan.digits, 256)), 256, 0, st, s.tcount, tiles, plan.digits, s.csum, chunks == 1 ? first_pos : nullptr);
         if (chunks > 1)
-          k_tile_scan_chunks<<<div_up(plan.digits, 8), 256, 0, st>>>(s.csum, chunks, plan.digits, first_pos);
+          launch_kernel(k_tile_scan_chunks, div_up(plan.digits, 8), 256, 0, st, s.csum, chunks, plan.digits, first_pos);
         cudaError_t e;
         if (first && last)
           e = launch_scatter<true, true>(kin, vin, n, kout, vout, shift, plan, s, count, st);
@@ -915,7 +913,7 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
     }
   }
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
-  return launch_exclusive_scan(count, start, nullptr, C, s.scan_status, s.counters, st);
+  return launch_start_scan(count, start, C, s, st);
 }
 
 cudaError_t radix_prepare() {
@@ -941,14 +939,12 @@ cudaError_t radix_prepare() {
 cudaError_t sort_run(const float4* pos, uint32_t n, const KeyFn& kf, uint64_t C, uint32_t* perm, uint32_t* start,
                      uint32_t* count, uint32_t* keys, uint32_t* overflow, const SortScratch& s, cudaStream_t st) {
   const RadixPlan plan = radix_plan(C);
-  if (cudaError_t e = cudaMemsetAsync(s.counters, 0, 4ull * kNumCounters, st); e != cudaSuccess) return e;
-  if (cudaError_t e = cudaMemsetAsync(s.digit_count, 0, 4ull * kRadixMaxPasses * kRadixMaxDigits, st);
-      e != cudaSuccess)
-    return e;
+  LinkedLaunches scope;
+  if (cudaError_t e = sort_state_zero(s, C, st); e != cudaSuccess) return e;
   uint32_t* ovf = overflow ? overflow : s.counters + kCounterOverflow;
   if (overflow)
     if (cudaError_t e = cudaMemsetAsync(overflow, 0, 4, st); e != cudaSuccess) return e;
-  launch_keys_digits(pos, n, kf, plan, keys, ovf, s, st);
+  launch_keys_digits(pos, n, kf, plan, keys, ovf, count, C, s, st);
   return launch_grid_sort(keys, n, C, plan, count, start, perm, s, st);
 }
 

@@ -89,16 +89,18 @@ size_t sort_scratch_bytes(uint32_t n, uint64_t C);
 // sort_scratch_zero clears its counters and counts (a fresh block once).
 void sort_scratch_carve(void* base, uint32_t n, uint64_t C, SortScratch* s);
 cudaError_t sort_scratch_zero(const SortScratch& s, cudaStream_t st);
+// Clears what a sort of C cells finds zeroed: the digit counts, the counters
+// and the scan's tile status (one memset, before the keys).
+cudaError_t sort_state_zero(const SortScratch& s, uint64_t C, cudaStream_t st);
 
 // Keys from float4 positions by element index, with the radix digit counts
-// of `plan` (s.digit_count must be zero) and the overflow flag.
+// of `plan`, the overflow flag, and count[C] zeroed.
 void launch_keys_digits(const float4* pos, uint32_t n, const KeyFn& kf, const RadixPlan& plan, uint32_t* keys,
-                        uint32_t* overflow, const SortScratch& s, cudaStream_t st);
+                        uint32_t* overflow, uint32_t* count, uint64_t C, const SortScratch& s, cudaStream_t st);
 
 // The sort proper from keys by element (keys[e] < C) whose digit counts are
-// in s.digit_count: writes perm[n], count[C] and start[C]. Clears what it
-// needs itself except s.digit_count (zeroed before the digit counts) and the
-// caller's error word.
+// in s.digit_count: writes perm[n], count[C] (zeroed by the key kernel) and
+// start[C], after sort_state_zero.
 cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan,
                              uint32_t* count, uint32_t* start, uint32_t* perm, const SortScratch& s,
                              cudaStream_t st);
@@ -139,17 +141,19 @@ __device__ __forceinline__ void digit_hist_flush(const uint32_t* sh, const Digit
     if (v) atomicAdd(h.global + (b / h.digits) * kRadixMaxDigits + b % h.digits, v);
   }
 }
+// The grid's threads together zero count[cells] (the key kernels).
+__device__ __forceinline__ void zero_counts(uint32_t* count, uint64_t cells) {
+  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += (uint64_t)gridDim.x * blockDim.x)
+    count[c] = 0u;
+}
 inline DigitHist digit_hist(const RadixPlan& p, const SortScratch& s) {
   return DigitHist{p.passes, p.width, p.digits, s.digit_count};
 }
-// Blocks of a grid-stride key kernel: enough to fill the GPU, few enough
-// that each block's histogram flush is cheap.
-uint32_t keys_grid(uint32_t n, uint32_t threads);
+// Blocks of a grid-stride key kernel over n elements that zeroes `cells`
+// counts: enough to fill the GPU, few enough that each block's histogram
+// flush is cheap.
+uint32_t keys_grid(uint32_t n, uint64_t cells, uint32_t threads);
 
-// Exclusive scan of n uint32 values (decoupled look-back); also zeroes
-// `zero_out` (n entries) when it is not null.
-cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t* zero_out, uint64_t n,
-                                  uint64_t* tile_status, uint32_t* counters, cudaStream_t st);
 uint32_t scan_tiles(uint64_t n);
 
 }  // namespace pf

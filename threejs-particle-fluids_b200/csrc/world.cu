@@ -35,6 +35,7 @@ namespace {
 
 // ---------------------------------------------------------- frame start ----
 __global__ void k_frame_start(WorldView V, uint32_t nscenes) {
+  pdl_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nscenes) return;
   const DevScene& S = V.scenes[s];
@@ -45,6 +46,7 @@ __global__ void k_frame_start(WorldView V, uint32_t nscenes) {
 
 // PrimitiveSet.ts:403-405, once per substep after friction.
 __global__ void k_tick(WorldView V, uint32_t nscenes, uint32_t sub) {
+  pdl_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nscenes) return;
   const DevScene& S = V.scenes[s];
@@ -57,6 +59,7 @@ __global__ void k_tick(WorldView V, uint32_t nscenes, uint32_t sub) {
 // positions (the grid window follows them; scenes past their substeps give
 // their unchanged ones). A 256-slot block belongs to one scene.
 __global__ void __launch_bounds__(kBlock) k_predict(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t s = scene_index(V, k);
   const DevScene& S = V.scenes[s];
@@ -78,6 +81,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(WorldView V, uint32_t sub) {
 // The cell bounds of every scene's predicted positions, where no predict
 // pass gathered them (the one-time init pass and the autotuner's sort).
 __global__ void __launch_bounds__(kBlock) k_bbox(WorldView V) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t s = scene_index(V, k);
   const DevScene& S = V.scenes[s];
@@ -90,6 +94,7 @@ __global__ void __launch_bounds__(kBlock) k_bbox(WorldView V) {
 // bounds are kept in bbox_last (the host widens windows between steps from
 // them) and reset for the next substep.
 __global__ void k_grid_fit(WorldView V, uint32_t nscenes) {
+  pdl_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nscenes) return;
   DevScene& S = V.scenes_rw[s];
@@ -129,6 +134,7 @@ __device__ __forceinline__ void advect_slot(const WorldView& V, const DevScene& 
   V.cur.x[k] = xs;
 }
 __global__ void __launch_bounds__(kBlock) k_advect(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const DevScene& S = scene_at(V, k);
@@ -137,6 +143,7 @@ __global__ void __launch_bounds__(kBlock) k_advect(WorldView V, uint32_t sub) {
 }
 // The advect of one group of run_groups, over its chunks.
 __global__ void __launch_bounds__(kBlock) k_advect_chunks(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);
@@ -150,9 +157,11 @@ __global__ void __launch_bounds__(kBlock) k_advect_chunks(WorldView V, uint32_t 
 // window, offset by the scene's key base; dead padding goes to the scene's
 // last key), with the radix digit counts of the sort in a block histogram
 // (grid-stride loop, one flush per block).
-__global__ void __launch_bounds__(kBlock) k_keys(WorldView V, DigitHist h) {
+__global__ void __launch_bounds__(kBlock) k_keys(WorldView V, DigitHist h, uint32_t cells) {
+  pdl_begin();
   extern __shared__ uint32_t sh[];
   digit_hist_zero(sh, h);
+  zero_counts(V.ccount, cells);
   __syncthreads();
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < V.n; k += gridDim.x * blockDim.x) {
     const uint32_t s = scene_index(V, k);
@@ -181,6 +190,7 @@ __global__ void __launch_bounds__(kBlock) k_keys(WorldView V, DigitHist h) {
 // Gather the per-slot state into cell order: new slot k takes particle
 // perm[k] from its old slot inv[perm[k]]; per-substep sums start at zero.
 __global__ void __launch_bounds__(kBlock) k_permute(WorldView V) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const uint32_t id = V.perm[k];
@@ -208,6 +218,7 @@ __global__ void __launch_bounds__(kBlock) k_permute(WorldView V) {
 
 // Without a grid the slots never move; only the per-substep sums reset.
 __global__ void __launch_bounds__(kBlock) k_reset_sums(WorldView V) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   V.cmask[k] = 0u;
@@ -219,6 +230,7 @@ __global__ void __launch_bounds__(kBlock) k_reset_sums(WorldView V) {
 // boundaryVolume.ts:36-52: V_i = 1 / max(sum_j W(x_i - x_j), 1e-12) over the
 // particle's own boundary range, walking the grid (not the neighbour list).
 __global__ void __launch_bounds__(kBlock) k_boundary_volume(WorldView V, uint32_t want_static, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const uint32_t b = tag_bnd(V.cur.tag[k]);
@@ -272,6 +284,7 @@ __device__ __forceinline__ const pf_primitive* stage_prims(const WorldView& V, P
 // the position pass, which applies them itself (k_s_delta).
 __global__ void __launch_bounds__(kBlock, 4) k_fluid_apply(WorldView V, uint32_t rank, uint32_t sub, uint32_t it,
                                                         uint32_t skip_homog) {
+  pdl_begin();
   // launched over the chunks of the scenes with a fluid (a block is one chunk)
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = g < V.n_fchunk * kSegAlign;
@@ -324,6 +337,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fluid_apply(WorldView V, uint32_t
 // velocity.ts:99-120: the vorticity confinement force eps (N x omega) dt with
 // N = eta / |eta| (eta from k_s_vort_grad, in dx), then the XSPH change.
 __global__ void __launch_bounds__(kBlock) k_xsph_apply(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -355,6 +369,7 @@ __global__ void __launch_bounds__(kBlock) k_xsph_apply(WorldView V, uint32_t ran
 // registers. Scenes whose last material is a fluid run this inside the
 // fluid's apply instead (collide_rank1).
 __global__ void __launch_bounds__(kBlock, 4) k_collide(WorldView V, uint32_t sub, uint32_t it) {
+  pdl_begin();
   // launched over the chunks of the scenes that need this pass (a block is
   // one chunk)
   static_assert(kBlock == kSegAlign, "one block per chunk");
@@ -379,6 +394,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_collide(WorldView V, uint32_t sub
 // PrimitiveSet.ts:367-398 with collider.ts:96-118, fused with the velocity
 // accumulator's apply (loop.ts:226-230).
 __global__ void __launch_bounds__(kBlock) k_friction(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   // A slot has work when a collider touched it this substep (the others'
   // multipliers are zero and add nothing) or contact friction
@@ -473,6 +489,7 @@ __global__ void __launch_bounds__(kBlock) k_friction(WorldView V, uint32_t sub) 
 // distance.ts:264-288 for one colour of constraints (no two share a particle).
 __global__ void __launch_bounds__(kBlock) k_cloth(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
                                                   uint32_t it) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const DevScene& S = V.scenes[V.c_scene[q]];
@@ -483,9 +500,14 @@ __global__ void __launch_bounds__(kBlock) k_cloth(WorldView V, uint32_t begin, u
   const float ws = wi + wj;
   const f3 off = xyz(xi) - xyz(xj);
   const float l = len(off);
-  if (ws <= 0.0f || l < 1e-12f) return;
+  // the multipliers start each substep at zero (so the first iteration does
+  // not read them)
+  const float lc = it ? V.c_lambda[q] : 0.0f;
+  if (ws <= 0.0f || l < 1e-12f) {
+    if (!it) V.c_lambda[q] = 0.0f;
+    return;
+  }
   const f3 nrm = off / l;
-  const float lc = V.c_lambda[q];
   const float at = V.c_comp[q] / (S.dt * S.dt);
   const float dl = (-(l - V.c_rest[q]) - at * lc) / (ws + at);
   V.cur.xs[i] = with_w(xyz(xi) + nrm * (wi * dl), wi);
@@ -499,6 +521,7 @@ __global__ void __launch_bounds__(kBlock) k_cloth(WorldView V, uint32_t begin, u
 // N1 = (p3 - p1) x (p3 - p2), N2 = (p4 - p2) x (p4 - p1), and the XPBD
 // multiplier update (xpbd.ts:26-36).
 __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const DevScene& S = V.scenes[V.b_scene[q]];
@@ -509,6 +532,8 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
   const f3 x1 = xyz(p1), x2 = xyz(p2), x3 = xyz(p3), x4 = xyz(p4);
   const f3 E = x2 - x1;
   const float e2 = dot(E, E);
+  const float lc = it ? V.b_lambda[q] : 0.0f;
+  if (!it) V.b_lambda[q] = 0.0f;  // for the returns below
   if (e2 < 1e-24f) return;
   const float el = sqrtf(e2);
   const f3 a3 = x3 - x1, b3 = x3 - x2;
@@ -529,7 +554,6 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
   const float w1 = p1.w, w2 = p2.w, w3 = p3.w, w4 = p4.w;
   const float sg = dot(g1, g1) * w1 + dot(g2, g2) * w2 + dot(g3, g3) * w3 + dot(g4, g4) * w4;
   if (sg <= 1e-30f) return;
-  const float lc = V.b_lambda[q];
   const float at = V.cloth_par[V.b_cloth[q]].bend_compliance / (S.dt * S.dt);
   const float dl = (-C - at * lc) / (sg + at);
   V.cur.xs[i1] = with_w(x1 + g1 * (w1 * dl), w1);
@@ -545,6 +569,7 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
 // its pinned anchor, read at its predicted position.
 __global__ void __launch_bounds__(kBlock) k_tether(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
                                                    uint32_t it) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const DevScene& S = V.scenes[V.t_scene[q]];
@@ -553,6 +578,8 @@ __global__ void __launch_bounds__(kBlock) k_tether(WorldView V, uint32_t begin, 
   const uint32_t i = V.inv[r.x];
   const float4 xi = V.cur.xs[i];
   const float w = xi.w;
+  const float lc = it ? V.t_lambda[q] : 0.0f;
+  if (!it) V.t_lambda[q] = 0.0f;  // for the returns below
   if (w <= 0.0f) return;
   const f3 d = xyz(xi) - xyz(V.cur.xs[V.inv[r.y]]);
   const float l = len(d);
@@ -562,7 +589,6 @@ __global__ void __launch_bounds__(kBlock) k_tether(WorldView V, uint32_t begin, 
     return;
   }
   if (l < 1e-12f) return;
-  const float lc = V.t_lambda[q];
   const float at = __uint_as_float(r.w) / (S.dt * S.dt);
   const float dl = (-(l - rest) - at * lc) / (w + at);
   V.cur.xs[i] = with_w(xyz(xi) + (d / l) * (w * dl), w);
@@ -574,6 +600,7 @@ __global__ void __launch_bounds__(kBlock) k_tether(WorldView V, uint32_t begin, 
 // particle (no scatter) from the committed positions and the velocities after
 // the prediction; the sum moves the predicted position by dt^2 w F.
 __global__ void __launch_bounds__(kBlock) k_aero(WorldView V, uint32_t begin, uint32_t end, uint32_t sub) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const uint2 rec = V.a_vtx[q];
@@ -613,6 +640,7 @@ __global__ void __launch_bounds__(kBlock) k_aero(WorldView V, uint32_t begin, ui
 // ClothSystem.ts:264-277: the mean velocity of each cloth particle's edge
 // neighbours, blended with its own (mix(v, mean, damping)).
 __global__ void __launch_bounds__(kBlock) k_damp_mean(WorldView V, uint32_t begin, uint32_t end, uint32_t sub) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const uint2 rec = V.d_vtx[q];
@@ -630,6 +658,7 @@ __global__ void __launch_bounds__(kBlock) k_damp_mean(WorldView V, uint32_t begi
 
 // ClothSystem.ts:278-284: particles with inverse mass > 0 take the blend.
 __global__ void __launch_bounds__(kBlock) k_damp_apply(WorldView V, uint32_t begin, uint32_t end, uint32_t sub) {
+  pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= end) return;
   const uint32_t k = V.inv[V.d_vtx[q].x];
@@ -639,6 +668,20 @@ __global__ void __launch_bounds__(kBlock) k_damp_apply(WorldView V, uint32_t beg
 }
 
 // ---------------------------------------------------------- soft bodies ----
+// A multiplier of the iteration before; zero in a substep's first iteration,
+// where every multiplier starts again (buildImplicitResetPairLambdaKernel),
+// so that nothing clears them in between.
+__device__ __forceinline__ float4 load_unless_first(const float4* p, uint32_t it) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(p), "r"(it));
+  return v;
+}
+
 __device__ __forceinline__ bool group_active(const WorldView& V, uint32_t g, uint32_t rank, uint32_t sub,
                                              uint32_t it, const DevSoft** D, const DevScene** S) {
   *D = &V.softs[V.grp_soft[g]];
@@ -648,6 +691,7 @@ __device__ __forceinline__ bool group_active(const WorldView& V, uint32_t g, uin
 
 // rotation.ts:297-314
 __global__ void __launch_bounds__(kBlock) k_rot_predict(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
   const DevSoft& D = V.softs[V.grp_soft[g]];
@@ -672,6 +716,7 @@ __global__ void __launch_bounds__(kBlock) k_rot_predict(WorldView V, uint32_t su
 
 // rotation.ts:316-343
 __global__ void __launch_bounds__(kBlock) k_rot_advect(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
   const DevSoft& D = V.softs[V.grp_soft[g]];
@@ -708,6 +753,7 @@ __global__ void __launch_bounds__(kBlock) k_rot_advect(WorldView V, uint32_t sub
 // the reference's centre pass does, and keeps it in registers; the members'
 // positions come back from cache for the moment.
 __global__ void __launch_bounds__(kBlock) k_sm_moment(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
   const DevSoft* D;
@@ -774,6 +820,7 @@ __global__ void __launch_bounds__(kBlock) k_sm_moment(WorldView V, uint32_t rank
 // past the last member, or whose member's body skips this pass, adds zero.
 template <uint32_t L>
 __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   static_assert(L == 1 || L == 2 || L == 4 || L == 8 || L == 16 || L == 32,
                 "lanes per member: a power of two dividing the warp");
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -818,7 +865,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
       const f3 c = mk(a0.w, a1.w, a2.w);
       const f3 cb = xyz(a3);
       const float at = a3.w / dt2;
-      const f3 lo = xyz(V.pair_lambda[m]);
+      const f3 lo = xyz(load_unless_first(V.pair_lambda + m, it));
       const f3 rr = rj - cb;
       const f3 goal = mk(dot(R0, rr), dot(R1, rr), dot(R2, rr)) + c;
       const f3 C = xyz(xj) - goal;
@@ -848,6 +895,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
 
 // shapeMatchImplicit.ts:325-401
 __global__ void __launch_bounds__(kBlock) k_sm_qp(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
   const DevSoft* D;
@@ -896,6 +944,7 @@ __global__ void __launch_bounds__(kBlock) k_sm_qp(WorldView V, uint32_t rank, ui
 // takes the polar decomposition.
 __global__ void __launch_bounds__(256) k_body_frame(WorldView V, uint32_t rank, uint32_t sub, uint32_t it,
                                                     uint32_t require_global) {
+  pdl_begin();
   const uint32_t b = blockIdx.x;
   if (b >= V.n_bodies) return;
   const DevBody B = V.bodies[b];
@@ -947,6 +996,7 @@ __global__ void __launch_bounds__(256) k_body_frame(WorldView V, uint32_t rank, 
 
 // shapeMatch.ts:277-351
 __global__ void __launch_bounds__(256) k_global_apply(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t b = blockIdx.x;
   if (b >= V.n_bodies) return;
   const DevBody B = V.bodies[b];
@@ -963,7 +1013,7 @@ __global__ void __launch_bounds__(256) k_global_apply(WorldView V, uint32_t rank
     const f3 goal = mk(dot(R0, ri), dot(R1, ri), dot(R2, ri)) + c;
     const float4 xs = V.cur.xs[sl];
     const f3 C = xyz(xs) - goal;
-    const f3 lo = xyz(V.lambda_g[id]);
+    const f3 lo = xyz(load_unless_first(V.lambda_g + id, it));
     const f3 dl = (neg(C) - lo * at) / (xs.w + at);
     V.lambda_g[id] = with_w(lo + dl, 0.0f);
     V.cur.xs[sl] = with_w(xyz(xs) + dl * xs.w, xs.w);
@@ -973,6 +1023,7 @@ __global__ void __launch_bounds__(256) k_global_apply(WorldView V, uint32_t rank
 // Positions by particle index for read-back: one thread per id.
 __global__ void __launch_bounds__(kBlock) k_gather_positions(WorldView V, const uint64_t* __restrict__ prefix,
                                                              float4* __restrict__ out) {
+  pdl_begin();
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= V.n) return;
   const uint32_t s = V.chunk_scene[id >> 8];
@@ -993,6 +1044,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_positions(WorldView V, const 
 // 2.5 and 1.9.
 __global__ void __launch_bounds__(kBlock) k_gather_rows(const uint32_t* __restrict__ inv, uint32_t cap,
                                                         const float4* __restrict__ src, float4* __restrict__ out) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cap) return;
   const float4 v = src[inv[i]];
@@ -1001,6 +1053,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_rows(const uint32_t* __restri
 __global__ void __launch_bounds__(kBlock) k_gather_words(const uint32_t* __restrict__ inv, uint32_t cap,
                                                          const float* __restrict__ src, uint32_t words, uint32_t word,
                                                          const uint32_t* __restrict__ tag, float* __restrict__ out) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cap) return;
   const uint32_t k = inv[i];
@@ -1010,6 +1063,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_words(const uint32_t* __restr
 // FluidSystem.ts:248-253: the impulse accumulator's apply over the fluid's
 // range, into the velocity and (times dt) the predicted position.
 __global__ void __launch_bounds__(kBlock) k_imp_apply(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -1035,6 +1089,7 @@ __global__ void __launch_bounds__(kBlock) k_imp_apply(WorldView V, uint32_t rank
 // Fresh slot maps (ids = inv = identity) and identity orientations.
 __global__ void __launch_bounds__(kBlock) k_init_slots(uint32_t* __restrict__ ids, uint32_t* __restrict__ inv,
                                                        float4* __restrict__ q, float4* __restrict__ qp, uint32_t n) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   ids[i] = i;
@@ -1052,6 +1107,7 @@ __global__ void __launch_bounds__(kBlock) k_import_scene(WorldView V, uint32_t s
                                                          const float* __restrict__ sbv, const uint32_t* __restrict__ sinv,
                                                          uint32_t sseg, const float4* __restrict__ sq,
                                                          const float4* __restrict__ som) {
+  pdl_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cap) return;
   const uint32_t from = sinv[sseg + i];
@@ -1076,7 +1132,7 @@ thread_local uint64_t t_launches = 0;
 template <typename K, typename... A>
 void launch_slots(K kernel, uint32_t n, cudaStream_t st, A... args) {
   if (n == 0) return;
-  kernel<<<div_up(n, kBlock), kBlock, 0, st>>>(args...);
+  launch_kernel(kernel, div_up(n, kBlock), kBlock, 0, st, args...);
   ++t_launches;
 }
 
@@ -2011,7 +2067,6 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   base_.max_tiles = (uint32_t)max_tiles;
   base_.n_grid_scenes = (uint32_t)grid_scene.size();
   base_.n_rows = row_base.back();
-  pair_entries_ = any_soft_local_ ? csr_idx.size() : 0;
   if (side_ok_) {
     PF_CUDA(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking));
     PF_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
@@ -2067,7 +2122,7 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   }
   // identity slot maps and orientations on the device; the scenes' own state
   // goes to their segments (scenes whose state is imported afterwards skip it)
-  k_init_slots<<<div_up(n_, kBlock), kBlock, 0, stream_>>>(base_.ids, base_.inv, base_.q, base_.qp, n_);
+  launch_kernel(k_init_slots, div_up(n_, kBlock), kBlock, 0, stream_, base_.ids, base_.inv, base_.q, base_.qp, n_);
   PF_CUDA(cudaGetLastError());
   {
     // pageable copies: the call returns once the source has been consumed,
@@ -2302,13 +2357,14 @@ pf_status World::wait_uploads() {
 
 void World::launch_frame_start_at(uint32_t parity) {
   const uint32_t K = (uint32_t)h_scenes_.size();
-  k_frame_start<<<div_up(K, 128), 128, 0, stream_>>>(view(parity), K);
+  launch_kernel(k_frame_start, div_up(K, 128), 128, 0, stream_, view(parity), K);
   ++t_launches;
 }
 
 // Cut the fluid scenes' grid rows into tiles and build the neighbour lists.
 void World::launch_tiles_build(const WorldView& V, uint32_t s) {
   cudaMemsetAsync(base_.tile_count, 0, 4, stream_);
+  break_link();
   launch_slots(k_build_tiles, base_.n_rows, stream_, V, s);
   launch_tiled(k_t_neighbors, kSmemNbr, V, s);
 }
@@ -2318,7 +2374,7 @@ template <typename K, typename... A>
 void World::launch_fluid(uint32_t block, K kernel, const WorldView& V, A... args) {
   const uint32_t slots = V.n_fchunk * kSegAlign;  // the view's chunks of scenes with a fluid
   if (!slots) return;
-  kernel<<<div_up(slots, block), block, 0, stream_>>>(V, args...);
+  launch_kernel(kernel, div_up(slots, block), block, 0, stream_, V, args...);
   ++t_launches;
 }
 
@@ -2755,7 +2811,7 @@ template <typename K, typename... A>
 void World::launch_tiled(K kernel, size_t smem, const WorldView& V, A... args) {
   const uint32_t grid = std::max<uint32_t>(
       1, std::min<uint32_t>(div_up(base_.max_tiles, kTileWarps), (uint32_t)sm_count() * 16));
-  kernel<<<grid, kTileThreads, smem, stream_>>>(V, args...);
+  launch_kernel(kernel, grid, kTileThreads, smem, stream_, V, args...);
   ++t_launches;
 }
 
@@ -2764,12 +2820,13 @@ void World::launch_tiled(K kernel, size_t smem, const WorldView& V, A... args) {
 void World::run_sort_and_permute(uint32_t parity, bool bbox_ready) {
   const WorldView V = view(parity);
   const uint32_t K = (uint32_t)h_scenes_.size();
-  if (!bbox_ready) launch_slots(k_bbox, n_, stream_, V);
-  k_grid_fit<<<div_up(K, 128), 128, 0, stream_>>>(V, K);
+  if (!bbox_ready) {
+    sort_state_zero(sort_, cells_, stream_);
+    launch_slots(k_bbox, n_, stream_, V);
+  }
+  launch_kernel(k_grid_fit, div_up(K, 128), 128, 0, stream_, V, K);
   ++t_launches;
-  cudaMemsetAsync(sort_.counters, 0, 4ull * kNumCounters, stream_);
-  cudaMemsetAsync(sort_.digit_count, 0, 4ull * kRadixMaxPasses * kRadixMaxDigits, stream_);
-  k_keys<<<keys_grid(n_, kBlock), kBlock, 4ull * radix_.passes * radix_.digits, stream_>>>(V, digit_hist(radix_, sort_));
+  launch_kernel(k_keys, keys_grid(n_, cells_, kBlock), kBlock, 4ull * radix_.passes * radix_.digits, stream_, V, digit_hist(radix_, sort_), cells_);
   launch_grid_sort(V.keys, n_, cells_, radix_, V.ccount, V.cstart, V.perm, sort_, stream_);
   t_launches += 1 + grid_sort_launches(radix_, n_);  // the keys, then the sort
   launch_slots(k_permute, n_, stream_, V);
@@ -2788,19 +2845,19 @@ void World::run_init_pass() {
 void World::launch_cloth_rank(const WorldView& V, uint32_t r, uint32_t s, uint32_t it, cudaStream_t st) {
   for (auto& rg : cloth_ranges_[r])
     if (rg.second > rg.first) {
-      k_cloth<<<div_up(rg.second - rg.first, kBlock), kBlock, 0, st>>>(V, rg.first, rg.second, s, it);
+      launch_kernel(k_cloth, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
       ++t_launches;
     }
   if (r < bend_ranges_.size())
     for (auto& rg : bend_ranges_[r])
       if (rg.second > rg.first) {
-        k_bend<<<div_up(rg.second - rg.first, kBlock), kBlock, 0, st>>>(V, rg.first, rg.second, s, it);
+        launch_kernel(k_bend, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
         ++t_launches;
       }
   if (r < teth_ranges_.size())
     for (auto& rg : teth_ranges_[r])
       if (rg.second > rg.first) {
-        k_tether<<<div_up(rg.second - rg.first, kBlock), kBlock, 0, st>>>(V, rg.first, rg.second, s, it);
+        launch_kernel(k_tether, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
         ++t_launches;
       }
 }
@@ -2808,12 +2865,13 @@ void World::launch_cloth_rank(const WorldView& V, uint32_t r, uint32_t s, uint32
 void World::launch_aero(const WorldView& V, uint32_t stage, uint32_t s) {
   const auto& rg = aero_ranges_[stage];
   if (rg.second <= rg.first) return;
-  k_aero<<<div_up(rg.second - rg.first, kBlock), kBlock, 0, stream_>>>(V, rg.first, rg.second, s);
+  launch_kernel(k_aero, div_up(rg.second - rg.first, kBlock), kBlock, 0, stream_, V, rg.first, rg.second, s);
   ++t_launches;
 }
 
 void World::run_substep(uint32_t s, uint32_t parity) {
   WorldView V = view(parity);
+  if (any_grid_) sort_state_zero(sort_, cells_, stream_);
   launch_slots(k_predict, n_, stream_, V, s);
   if (any_soft_local_) launch_slots(k_rot_predict, base_.n_grp, stream_, V, s);
   if (any_grid_) {
@@ -2828,8 +2886,8 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   // preSolve: contacts first (loop.ts:196-223), then the materials'
   if (any_contact_) {
     const uint32_t K = (uint32_t)h_scenes_.size();
-    k_con_gen<<<n_ / kBlock, kBlock, 0, stream_>>>(V, s);
-    k_con_scan<<<K, 1024, 0, stream_>>>(V, s);
+    launch_kernel(k_con_gen, n_ / kBlock, kBlock, 0, stream_, V, s);
+    launch_kernel(k_con_scan, K, 1024, 0, stream_, V, s);
     launch_slots(k_con_stab, n_, stream_, V, s);
     launch_slots(k_con_apply2, n_, stream_, V, s);
     t_launches += 2;
@@ -2851,12 +2909,6 @@ void World::run_substep(uint32_t s, uint32_t parity) {
       launch_slots(k_imp_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s);
     }
   launch_aero(V, 1, s);
-  // pair multipliers reset every substep (buildImplicitResetPairLambdaKernel)
-  if (any_soft_local_ && pair_entries_) cudaMemsetAsync(base_.pair_lambda, 0, 16ull * pair_entries_, stream_);
-  if (any_soft_global_) cudaMemsetAsync(base_.lambda_g, 0, 16ull * n_, stream_);
-  if (base_.n_cons) cudaMemsetAsync(base_.c_lambda, 0, 4ull * base_.n_cons, stream_);
-  if (base_.n_bend) cudaMemsetAsync(base_.b_lambda, 0, 4ull * base_.n_bend, stream_);
-  if (base_.n_teth) cudaMemsetAsync(base_.t_lambda, 0, 4ull * base_.n_teth, stream_);
   // iterations
   // Cloth-only scenes (and material-free scenes with colliders) share no
   // slot with the others: their colour sweeps and collider passes run on a
@@ -2865,6 +2917,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   if (fork) {
     cudaEventRecord(ev_fork_, stream_);
     cudaStreamWaitEvent(side_stream_, ev_fork_, 0);
+    break_link();
     for (uint32_t it = 0; it < max_iter_; ++it) {
       for (uint32_t r = 0; r < cloth_ranges_.size(); ++r) launch_cloth_rank(V, r, s, it, side_stream_);
       if (any_contact_) launch_slots(k_con_solve, n_, side_stream_, V, s, it);
@@ -2893,19 +2946,19 @@ void World::run_substep(uint32_t s, uint32_t parity) {
         launch_slots(k_sm_moment, base_.n_grp, stream_, V, r, s, it);
         if (base_.n_mem_ids) {  // mem_lanes_ lanes per cluster member
           const uint32_t grid = (uint32_t)(((uint64_t)mem_lanes_ * base_.n_mem_ids + kBlock - 1) / kBlock);
-          if (mem_lanes_ == 1) k_sm_gather<1><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
-          else if (mem_lanes_ == 2) k_sm_gather<2><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
-          else if (mem_lanes_ == 4) k_sm_gather<4><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
-          else if (mem_lanes_ == 8) k_sm_gather<8><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
-          else if (mem_lanes_ == 16) k_sm_gather<16><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
-          else k_sm_gather<32><<<grid, kBlock, 0, stream_>>>(V, r, s, it);
+          if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 2) launch_kernel(k_sm_gather<2>, grid, kBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 4) launch_kernel(k_sm_gather<4>, grid, kBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 8) launch_kernel(k_sm_gather<8>, grid, kBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 16) launch_kernel(k_sm_gather<16>, grid, kBlock, 0, stream_, V, r, s, it);
+          else launch_kernel(k_sm_gather<32>, grid, kBlock, 0, stream_, V, r, s, it);
           ++t_launches;
         }
         launch_slots(k_sm_qp, base_.n_grp, stream_, V, r, s, it);
       }
       if (has_global && base_.n_bodies) {
-        k_body_frame<<<base_.n_bodies, 256, 0, stream_>>>(V, r, s, it, 1u);
-        k_global_apply<<<base_.n_bodies, 256, 0, stream_>>>(V, r, s, it);
+        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, it, 1u);
+        launch_kernel(k_global_apply, base_.n_bodies, 256, 0, stream_, V, r, s, it);
         t_launches += 2;
       }
       if (!fork && r < cloth_ranges_.size()) launch_cloth_rank(V, r, s, it, stream_);
@@ -2916,6 +2969,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   if (fork) {
     cudaEventRecord(ev_join_, side_stream_);
     cudaStreamWaitEvent(stream_, ev_join_, 0);
+    break_link();
   }
   launch_slots(k_advect, n_, stream_, V, s);
   for (uint32_t r = 0; r < max_rank_; ++r) {
@@ -2933,15 +2987,15 @@ void World::run_substep(uint32_t s, uint32_t parity) {
     if (has_local) {
       launch_slots(k_rot_advect, base_.n_grp, stream_, V, s);
       if (base_.n_bodies) {
-        k_body_frame<<<base_.n_bodies, 256, 0, stream_>>>(V, r, s, 0u, 0u);
+        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, 0u, 0u);
         ++t_launches;
       }
     }
     if (r < damp_ranges_.size() && damp_ranges_[r].second > damp_ranges_[r].first) {
       const auto& rg = damp_ranges_[r];
       const uint32_t g = div_up(rg.second - rg.first, kBlock);
-      k_damp_mean<<<g, kBlock, 0, stream_>>>(V, rg.first, rg.second, s);
-      k_damp_apply<<<g, kBlock, 0, stream_>>>(V, rg.first, rg.second, s);
+      launch_kernel(k_damp_mean, g, kBlock, 0, stream_, V, rg.first, rg.second, s);
+      launch_kernel(k_damp_apply, g, kBlock, 0, stream_, V, rg.first, rg.second, s);
       t_launches += 2;
     }
   }
@@ -2951,7 +3005,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   if (any_prims_ || any_contact_) launch_slots(k_friction, n_, stream_, V, s);
   if (any_prims_) {
     const uint32_t K = (uint32_t)h_scenes_.size();
-    k_tick<<<div_up(K, 128), 128, 0, stream_>>>(V, K, s);
+    launch_kernel(k_tick, div_up(K, 128), 128, 0, stream_, V, K, s);
     ++t_launches;
   }
 }
@@ -2974,6 +3028,7 @@ pf_status World::step(double dt) {
   }
   const uint32_t flips = any_grid_ ? (max_sub_ & 1u) : 0u;
   auto body = [&](uint32_t p0) {
+    LinkedLaunches scope;
     t_launches = 0;
     launch_frame_start_at(p0);
     uint32_t p = p0;
@@ -3404,7 +3459,7 @@ pf_status World::import_scene(uint32_t s, const World& src, uint32_t src_s) {
   if (S.cap == 0) return PF_OK;
   const StateBuf& B = src.buf_[src.parity_];
   const WorldView V = view(parity_);
-  k_import_scene<<<div_up(S.cap, kBlock), kBlock, 0, stream_>>>(V, S.seg_start, S.cap, B.x, B.v, B.bv, src.base_.inv,
+  launch_kernel(k_import_scene, div_up(S.cap, kBlock), kBlock, 0, stream_, V, S.seg_start, S.cap, B.x, B.v, B.bv, src.base_.inv,
                                                                  T.seg_start, src.base_.q, src.base_.omega);
   PF_CUDA(cudaGetLastError());
   return PF_OK;

@@ -631,7 +631,6 @@ class World {
   DevSdf* h_pinned_sdfs_ = nullptr;
   DevCloth* h_pinned_cloth_ = nullptr;
   bool prims_dirty_ = true;
-  size_t pair_entries_ = 0;
   float4* stage_pos_ = nullptr;  // gather buffer of read_positions
   float4* stage_pos2_ = nullptr;  // the second one of read_positions_async
   cudaStream_t read_stream_ = nullptr;  // copies of read_positions_async (made on first use)

@@ -60,6 +60,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* ws, ui
 // two emitting slots is kept by the lower slot. The block is one 256-slot
 // chunk: it also forms the slots' prefix inside the chunk and the chunk's sum.
 __global__ void __launch_bounds__(kBlock) k_con_gen(WorldView V, uint32_t sub) {
+  pdl_begin();
   __shared__ uint32_t ws[32];
   const uint32_t k = blockIdx.x * kBlock + threadIdx.x;  // the grid covers n exactly
   const DevScene& S = scene_at(V, k);
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(kBlock) k_con_gen(WorldView V, uint32_t sub) {
 // The chunks' first pair index inside their scene (one block per scene), and
 // the scene's pair count of this substep (ContactBuffer.counter).
 __global__ void __launch_bounds__(1024) k_con_scan(WorldView V, uint32_t sub) {
+  pdl_begin();
   __shared__ uint32_t ws[32];
   const DevScene& S = V.scenes[blockIdx.x];
   if (!S.contact || sub >= S.substeps) return;
@@ -145,6 +147,7 @@ __device__ __forceinline__ uint32_t con_live(const WorldView& V, const DevScene&
 // separated, the change going to both the committed and the predicted
 // positions (applied by k_con_apply2).
 __global__ void __launch_bounds__(kBlock) k_con_stab(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const DevScene& S = scene_at(V, k);
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(kBlock) k_con_stab(WorldView V, uint32_t sub) 
 
 // accumulator.ts:101-131 over [positions, predictedPositions] (loop.ts:393).
 __global__ void __launch_bounds__(kBlock) k_con_apply2(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const uint32_t s = scene_index(V, k);
@@ -189,6 +193,7 @@ __global__ void __launch_bounds__(kBlock) k_con_apply2(WorldView V, uint32_t sub
 // friction inside the cone lambda_t <= mu_s lambda_n, scattered into the
 // position sums that the collider pass applies.
 __global__ void __launch_bounds__(kBlock) k_con_solve(WorldView V, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const DevScene& S = scene_at(V, k);
@@ -230,6 +235,7 @@ __global__ void __launch_bounds__(kBlock) k_con_solve(WorldView V, uint32_t sub,
 // reduced by at most mu_k lambda_n / dt, into the velocity sums that the
 // friction pass applies.
 __global__ void __launch_bounds__(kBlock) k_con_friction(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= V.n) return;
   const DevScene& S = scene_at(V, k);

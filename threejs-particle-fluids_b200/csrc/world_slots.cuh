@@ -25,24 +25,25 @@
 namespace pf {
 
 // A list entry, or 2, 4 or 8 16-bit entries of one group (read-only for the
-// kernel). A miss fetches 256 bytes into L2: with the warp-blocked layout
-// that is the warp's neighbouring entries too.
+// kernel; volatile, so that none moves ahead of pdl_begin()). A miss fetches
+// 256 bytes into L2: with the warp-blocked layout that is the warp's
+// neighbouring entries too.
 __device__ __forceinline__ uint32_t ld_entry(const uint32_t* p) {
   uint32_t v;
-  asm("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 template <uint32_t kN>
 __device__ __forceinline__ void ld_group(const uint16_t* p, uint32_t (&w)[kN / 2]) {
   static_assert(kN == 2 || kN == 4 || kN == 8, "2, 4 or 8 entries");
   if constexpr (kN == 8)
-    asm("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
         : "l"(p));
   else if constexpr (kN == 4)
-    asm("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
+    asm volatile("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
   else
-    asm("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(w[0]) : "l"(p));
+    asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(w[0]) : "l"(p));
 }
 
 // The list of slot k: its warp's base (kNbrWide: 32-bit entries) and the
@@ -233,6 +234,7 @@ __device__ __forceinline__ void lambda_terms(const DevFluid& F, f3 xi, float4 xj
 // order; the autotuner picks the faster form).
 template <uint32_t kNbrUnroll, bool kDens, bool kFlat>
 __global__ void k_s_neighbors(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;     // whole warps
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -424,6 +426,7 @@ __global__ void k_s_neighbors(WorldView V, uint32_t sub) {
 // lambda.ts:41-71
 template <uint32_t kNbrUnroll>
 __global__ void __maxnreg__(kNbrUnroll == 8 ? 80 : 48) k_s_lambda(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -465,6 +468,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 80 : 48) k_s_lambda(WorldView V, u
 // is rewritten in place; the arithmetic is that of the separate apply.
 template <uint32_t kNbrUnroll, bool kReact>
 __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, uint32_t rank, uint32_t sub, uint32_t it, uint32_t apply) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -543,6 +547,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, ui
 // confinement, the curl omega = sum V_j (v_i - v_j) x grad W.
 template <uint32_t kNbrUnroll, bool kBnd>
 __global__ void k_s_xsph(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -590,6 +595,7 @@ __global__ void k_s_xsph(WorldView V, uint32_t rank, uint32_t sub) {
 // grad W (|omega_j| - |omega_i|) V, into dx (free after the iterations).
 template <uint32_t kNbrUnroll>
 __global__ void k_s_vort_grad(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -619,6 +625,7 @@ __global__ void k_s_vort_grad(WorldView V, uint32_t rank, uint32_t sub) {
 // substep's predicted positions.
 template <uint32_t kNbrUnroll>
 __global__ void k_s_color_normal(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
@@ -662,6 +669,7 @@ __device__ __forceinline__ float adhesion_spline(float r, const DevFluid& F) {
 // neighbours on the fluid side only; both as fixed-point velocity changes.
 template <uint32_t kNbrUnroll>
 __global__ void k_s_impulses(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid

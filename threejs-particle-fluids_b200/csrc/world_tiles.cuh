@@ -79,6 +79,7 @@ __device__ __forceinline__ int32_t next_tile(const DevScene& S, const uint32_t* 
 // Cut every grid row of the fluid scenes into tiles: one thread per row,
 // counted first, one atomic per warp for the warp's tile range, then emitted.
 __global__ void __launch_bounds__(kBlock) k_build_tiles(WorldView V, uint32_t sub) {
+  pdl_begin();
   const uint32_t R = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31u;
   bool valid = R < V.n_rows;
@@ -195,21 +196,22 @@ __device__ __forceinline__ void stage_rows(const WarpTile& W, const E* __restric
 // Visit a particle's list entries in order, fetching four halo indices per
 // round so their loads overlap.
 template <typename Fn>
-__device__ __forceinline__ void for_each_h(const uint16_t* __restrict__ nl, size_t n, uint32_t cnt, Fn&& one) {
+__device__ __forceinline__ void for_each_h(const uint16_t* nl, size_t n, uint32_t cnt, Fn&& one) {
   uint32_t m = 0;
   for (; m + 4 <= cnt; m += 4) {
     uint32_t h[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) h[q] = __ldg(nl + (m + q) * n);
+    for (int q = 0; q < 4; ++q) h[q] = nl[(m + q) * n];
 #pragma unroll
     for (int q = 0; q < 4; ++q) one(h[q]);
   }
-  for (; m < cnt; ++m) one(__ldg(nl + m * n));
+  for (; m < cnt; ++m) one(nl[m * n]);
 }
 
 // neighborList.ts:48-71 over warp tiles: candidates are the 27 cells of the
 // particle's own cell; entries are halo indices of the tile.
 __global__ void __launch_bounds__(kTileThreads) k_t_neighbors(WorldView V, uint32_t sub) {
+  pdl_begin();
   extern __shared__ float4 smem4[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float4* hx = smem4 + warp * kWarpHalo;
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(kTileThreads) k_t_neighbors(WorldView V, uint3
 
 // lambda.ts:41-71 over warp tiles.
 __global__ void __launch_bounds__(kTileThreads) k_t_lambda(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   extern __shared__ float4 smem4[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float4* hx = smem4 + warp * kWarpHalo;
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(kTileThreads) k_t_lambda(WorldView V, uint32_t
 // positionDelta.ts:41-85 over warp tiles (the reaction on dynamic boundary
 // neighbours goes into the fixed-point reaction sums by slot).
 __global__ void __launch_bounds__(kTileThreads) k_t_delta(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+  pdl_begin();
   extern __shared__ float4 smem4[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float4* hx = smem4 + warp * kWarpHalo;
@@ -400,6 +404,7 @@ __global__ void __launch_bounds__(kTileThreads) k_t_delta(WorldView V, uint32_t 
 
 // velocity.ts:43-70 (XSPH) over warp tiles: committed positions and velocities.
 __global__ void __launch_bounds__(kTileThreads) k_t_xsph(WorldView V, uint32_t rank, uint32_t sub) {
+  pdl_begin();
   extern __shared__ float4 smem4[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float4* hx = smem4 + warp * kWarpHalo;
