@@ -243,14 +243,25 @@ __global__ void __launch_bounds__(kBlock) k_boundary_volume(WorldView V, uint32_
   const float4* pos = want_static ? V.cur.x : V.cur.xs;
   const f3 xi = xyz(pos[k]);
   float sum = 0.0f;
-  walk27(S, V.cstart, V.ccount, xi, [&](uint32_t j) {
-    const uint32_t idj = V.ids[j];
-    if (idj < B.start || idj >= B.start + B.count) return true;
-    const f3 off = xi - xyz(pos[j]);
-    const float rsq = dot(off, off);
-    if (rsq >= F.hsq) return true;
-    sum += poly6(rsq, F);
-    return true;
+  walk27_rows(S, V.cstart, V.ccount, xi, [&](uint32_t j, uint32_t e) {
+    // four candidates' loads in flight, summed in walk order
+    for (; j < e; j += 4) {
+      uint32_t id[4];
+      float4 x[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (j + q < e) {
+          id[q] = V.ids[j + q];
+          x[q] = pos[j + q];
+        }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (j + q >= e || id[q] - B.start >= B.count) continue;
+        const f3 off = xi - xyz(x[q]);
+        const float rsq = dot(off, off);
+        if (rsq < F.hsq) sum += poly6(rsq, F);
+      }
+    }
   });
   const float bv = 1.0f / fmaxf(sum, 1e-12f);
   V.cur.bv[k] = bv;

@@ -231,29 +231,27 @@ __device__ __forceinline__ void bbox_block_add(const WorldView& V, const DevScen
 // Visit the sorted slots of the 27 cells around p in the reference's order
 // (query.ts:37-66: dz, dy, dx; within a cell ascending particle index). With
 // linear keys the three cells of one (dy, dz) row are consecutive keys, so a
-// row is one contiguous slot range. fn(slot) returns false to stop early.
+// row is one contiguous slot range: row(first, end) per row.
 template <typename F>
-__device__ __forceinline__ void walk27(const DevScene& S, const uint32_t* __restrict__ cstart,
-                                       const uint32_t* __restrict__ ccount, f3 p, F&& fn) {
+__device__ __forceinline__ void walk27_rows(const DevScene& S, const uint32_t* __restrict__ cstart,
+                                            const uint32_t* __restrict__ ccount, f3 p, F&& row) {
   int32_t cx, cy, cz;
   local_cell(S, p, &cx, &cy, &cz, nullptr);
   const int32_t x0 = max(cx - 1, 0), x1 = min(cx + 1, (int32_t)S.dims[0] - 1);
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int32_t z = cz + dz;
-    if (z < 0 || z >= (int32_t)S.dims[2]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int32_t y = cy + dy;
-      if (y < 0 || y >= (int32_t)S.dims[1]) continue;
-      const uint32_t row = S.cell_base + S.dims[0] * ((uint32_t)y + S.dims[1] * (uint32_t)z);
-      const uint32_t k0 = row + (uint32_t)x0, k1 = row + (uint32_t)x1;
-      const uint32_t s0 = __ldg(cstart + k0);
-      const uint32_t s1 = __ldg(cstart + k1) + __ldg(ccount + k1);
-      for (uint32_t j = s0; j < s1; ++j)
-        if (!fn(j)) return;
-    }
+  // the rows' ranges first, their loads in flight together
+  uint32_t rs[9], re[9];
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int32_t z = cz + r / 3 - 1, y = cy + r % 3 - 1;
+    rs[r] = re[r] = 0;
+    if (z < 0 || z >= (int32_t)S.dims[2] || y < 0 || y >= (int32_t)S.dims[1]) continue;
+    const uint32_t at = S.cell_base + S.dims[0] * ((uint32_t)y + S.dims[1] * (uint32_t)z);
+    rs[r] = __ldg(cstart + at + x0);
+    re[r] = __ldg(cstart + at + x1) + __ldg(ccount + at + x1);
   }
+#pragma unroll
+  for (int r = 0; r < 9; ++r) row(rs[r], re[r]);
 }
-
 // ------------------------------------------------------------ quaternions ----
 __device__ __forceinline__ f3 qrot(float4 q, f3 v) {
   const f3 qv = mk(q.x, q.y, q.z);

@@ -506,11 +506,17 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, ui
     const f3 g = off * (shape * -F.spiky);
 #endif
     if (react && bvj > 0.0f && xj.w > 0.0f) {
-      const uint32_t idj = V.ids[j];
-      bool in = false;
-      for (uint32_t b = 0; b < F.bnd_count; ++b) {
-        const DevBoundary B = V.bnds[F.bnd_first + b];
-        in = in || (idj >= B.start && idj < B.start + B.count);
+      // Is j on one of this fluid's boundaries? Its tag names the last added
+      // boundary that holds it (zero: none does), which decides unless that
+      // one is another fluid's; only then the fluid's ranges are searched.
+      const uint32_t tb = tag_bnd(__ldg(V.cur.tag + j));
+      bool in = tb != 0 && tb - 1u - F.bnd_first < F.bnd_count;
+      if (tb != 0 && !in) {
+        const uint32_t idj = V.ids[j];
+        for (uint32_t b = 0; b < F.bnd_count; ++b) {
+          const DevBoundary B = V.bnds[F.bnd_first + b];
+          in = in || (idj >= B.start && idj < B.start + B.count);
+        }
       }
       if (in) acc_add(V.acc_react, j, g * (-(li / F.rho0) * (F.rho0 * bvj) * xj.w), F.react_scale);
     }
