@@ -93,3 +93,37 @@ def test_plain_steps_as_graph_same_bits(pfsim, substeps):
             assert np.array_equal(a.readback(f), b.readback(0, f)), k
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("wide", [0, 1])
+@pytest.mark.parametrize("unroll", [2, 4, 8])
+@pytest.mark.parametrize("per_cell", [1, 3, 8, 30, 70])
+def test_list_build_columns(oracle, monkeypatch, per_cell, unroll, wide):
+    """The neighbour list where a lane's column of hits stays nearly empty, is
+    filled in the last rows, and overflows (64 entries at most, the rest
+    flagged), with 16- and 32-bit entries: the oracle's lists, element for
+    element."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    monkeypatch.setenv("PFSIM_NBR_PATH", "0")
+    monkeypatch.setenv("PFSIM_SLOT_BLOCK", "128")
+    monkeypatch.setenv("PFSIM_SLOT_UNROLL", str(unroll))
+    monkeypatch.setenv("PFSIM_NBR_WIDE", str(wide))
+    h = 0.04
+    r = np.random.default_rng(per_cell)
+    n = 125 * per_cell + 7
+    pos = r.uniform(0.2, 0.2 + 5 * h, (n, 3)).astype(np.float32)
+    rec = R.Recipe(capacity=n, radius=0.005, uploads=[R.Upload(0, pos)],
+                   materials=[("fluid", R.FluidOpts(range=(0, n), particle_spacing=0.02, smoothing_radius=h,
+                                                    rest_density=1000.0, viscosity=0.01))],
+                   loop=R.LoopOpts(substeps=1, iterations=1, gravity=(0.0, 0.0, 0.0)))
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    a.step(1 / 60)
+    b.step(1 / 60)
+    for f in (N.PF_FIELD_NEIGHBOR_COUNT, N.PF_FIELD_NEIGHBORS):
+        assert np.array_equal(a.readback(f), b.readback(f))
+    assert a.overflow()["neighbors"] == b.overflow()["neighbors"] == (per_cell == 70 or per_cell == 30)
+    # densities: sums of at most 64 positive terms, each rounded a few times
+    np.testing.assert_allclose(a.readback(N.PF_FIELD_DENSITY), b.readback(N.PF_FIELD_DENSITY), rtol=2e-5)
+    a.close()

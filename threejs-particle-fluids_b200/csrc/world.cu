@@ -1152,18 +1152,26 @@ size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 // The slot neighbour passes use no shared memory and gather their
 // neighbours' records through L1: each asks for the largest L1 (a hint the
 // runtime may round), once per device, outside any stream capture.
+constexpr int kHitCarveout = 45;  // per cent of an SM's shared memory (the list build)
 template <typename K>
 cudaError_t prefer_l1(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxL1);
+}
+// The list build's hit columns: up to 512 threads a block, and a carve-out
+// that leaves the gathers the larger half.
+template <typename K>
+cudaError_t allow_hits(K kernel) {
+  if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(512 * kHitBytes));
+      e != cudaSuccess)
+    return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kHitCarveout);
 }
 template <uint32_t U>
 cudaError_t prefer_l1_depth() {
   cudaError_t e = cudaSuccess;
   auto on = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-  on(prefer_l1(k_s_neighbors<U, false, false>));
-  on(prefer_l1(k_s_neighbors<U, true, false>));
-  on(prefer_l1(k_s_neighbors<U, false, true>));
-  on(prefer_l1(k_s_neighbors<U, true, true>));
+  on(allow_hits(k_s_neighbors<U, false>));
+  on(allow_hits(k_s_neighbors<U, true>));
   on(prefer_l1(k_s_lambda<U>));
   on(prefer_l1(k_s_delta<U, false>));
   on(prefer_l1(k_s_delta<U, true>));
@@ -2383,9 +2391,13 @@ void World::launch_tiles_build(const WorldView& V, uint32_t s) {
 // One-thread-per-slot fluid kernels at a tuned block size.
 template <typename K, typename... A>
 void World::launch_fluid(uint32_t block, K kernel, const WorldView& V, A... args) {
+  launch_fluid_smem(block, 0, kernel, V, args...);
+}
+template <typename K, typename... A>
+void World::launch_fluid_smem(uint32_t block, size_t smem, K kernel, const WorldView& V, A... args) {
   const uint32_t slots = V.n_fchunk * kSegAlign;  // the view's chunks of scenes with a fluid
   if (!slots) return;
-  launch_kernel(kernel, div_up(slots, block), block, 0, stream_, V, args...);
+  launch_kernel(kernel, div_up(slots, block), block, smem, stream_, V, args...);
   ++t_launches;
 }
 
@@ -2399,23 +2411,19 @@ void World::launch_fluid(uint32_t block, K kernel, const WorldView& V, A... args
   } while (0)
 // The list build, forming the first iteration's density and lambda of
 // first-material fluids when nothing moves between the two (fuse_dens_).
-#define PF_NBR_FLAT(FLAT, ...)                                                          \
-  do {                                                                                  \
-    const uint32_t b_ = tune_.block[kSlotNbr], u_ = tune_.unroll[kSlotNbr];             \
-    if (fuse_dens_) {                                                                   \
-      if (u_ == 2) launch_fluid(b_, k_s_neighbors<2, true, FLAT>, __VA_ARGS__);         \
-      else if (u_ == 8) launch_fluid(b_, k_s_neighbors<8, true, FLAT>, __VA_ARGS__);    \
-      else launch_fluid(b_, k_s_neighbors<4, true, FLAT>, __VA_ARGS__);                 \
-    } else {                                                                            \
-      if (u_ == 2) launch_fluid(b_, k_s_neighbors<2, false, FLAT>, __VA_ARGS__);        \
-      else if (u_ == 8) launch_fluid(b_, k_s_neighbors<8, false, FLAT>, __VA_ARGS__);   \
-      else launch_fluid(b_, k_s_neighbors<4, false, FLAT>, __VA_ARGS__);                \
-    }                                                                                   \
-  } while (0)
 #define PF_NBR(...)                                                                     \
   do {                                                                                  \
-    if (tune_.nbr_flat) PF_NBR_FLAT(true, __VA_ARGS__);                                 \
-    else PF_NBR_FLAT(false, __VA_ARGS__);                                               \
+    const uint32_t b_ = tune_.block[kSlotNbr], u_ = tune_.unroll[kSlotNbr];             \
+    const size_t m_ = (size_t)b_ * kHitBytes;                                           \
+    if (fuse_dens_) {                                                                   \
+      if (u_ == 2) launch_fluid_smem(b_, m_, k_s_neighbors<2, true>, __VA_ARGS__);      \
+      else if (u_ == 8) launch_fluid_smem(b_, m_, k_s_neighbors<8, true>, __VA_ARGS__); \
+      else launch_fluid_smem(b_, m_, k_s_neighbors<4, true>, __VA_ARGS__);              \
+    } else {                                                                            \
+      if (u_ == 2) launch_fluid_smem(b_, m_, k_s_neighbors<2, false>, __VA_ARGS__);     \
+      else if (u_ == 8) launch_fluid_smem(b_, m_, k_s_neighbors<8, false>, __VA_ARGS__);\
+      else launch_fluid_smem(b_, m_, k_s_neighbors<4, false>, __VA_ARGS__);             \
+    }                                                                                   \
   } while (0)
 // XSPH, without the boundary-volume gather when the world has no boundaries.
 #define PF_XSPH(...)                                                                    \
@@ -2531,7 +2539,8 @@ void World::run_groups(const WorldView& V, uint32_t s, bool apply) {
 
 // Tuning cache. With PFSIM_TUNE_CACHE naming a file, the tuner first looks
 // there for a line
-//   pfsim-tune-1 <gpu> <sms> <config> <n> <path> <block x4> <unroll x4> <group> <flat> <wide>
+//   pfsim-tune-1 <gpu> <sms> <config> <n> <path> <block x4> <unroll x4> <group> <0 or 1> <wide>
+// (the field before the last chose between two list walks and is not used)
 // keyed by the GPU (its name, blanks as '_', and its SM count), the world's
 // configuration (a 64-bit FNV-1a hash, in hex, of its scenes' capacities,
 // substeps, iterations, build-time grid windows, fluids and contacts, and
@@ -2587,8 +2596,8 @@ bool World::load_tuning(const char* file, const std::string& key) {
   if (!f) return false;
   uint64_t pure_total = 0;
   for (uint64_t p : pure_parts_) pure_total += p;
-  auto valid = [&](const Tuning& t) {
-    if (t.path > 1 || t.nbr_flat > 1 || t.nbr_wide > 1) return false;
+  auto valid = [&](const Tuning& t, uint32_t flat) {
+    if (t.path > 1 || flat > 1 || t.nbr_wide > 1) return false;
     if (t.path == 1 && (any_vort_ || any_imp_ || any_multi_fluid_)) return false;
     for (int q = 0; q < 4; ++q) {
       const uint32_t b = t.block[q], u = t.unroll[q];
@@ -2604,15 +2613,15 @@ bool World::load_tuning(const char* file, const std::string& key) {
   while (std::fgets(line, sizeof line, f)) {
     char tag[32], gpu[256], cfg[32];
     int sms = 0;
-    unsigned n = 0;
+    unsigned n = 0, flat = 0;
     Tuning t;
     const int got = std::sscanf(line, "%31s %255s %d %31s %u %u %u %u %u %u %u %u %u %u %u %u %u", tag, gpu, &sms, cfg, &n,
                                 &t.path, &t.block[0], &t.block[1], &t.block[2], &t.block[3], &t.unroll[0], &t.unroll[1],
-                                &t.unroll[2], &t.unroll[3], &t.group, &t.nbr_flat, &t.nbr_wide);
+                                &t.unroll[2], &t.unroll[3], &t.group, &flat, &t.nbr_wide);
     if (got != 17 || std::strcmp(tag, "pfsim-tune-1") != 0) continue;
     char k[320];
     std::snprintf(k, sizeof k, "%s %d %s %u", gpu, sms, cfg, n);
-    if (key != k || !valid(t)) continue;
+    if (key != k || !valid(t, flat)) continue;
     hit = t;
     found = true;
   }
@@ -2626,7 +2635,7 @@ void World::store_tuning(const char* file, const std::string& key) const {
   const Tuning& t = tune_;
   const int len = std::snprintf(line, sizeof line, "pfsim-tune-1 %s %u %u %u %u %u %u %u %u %u %u %u %u\n", key.c_str(),
                                 t.path, t.block[0], t.block[1], t.block[2], t.block[3], t.unroll[0], t.unroll[1],
-                                t.unroll[2], t.unroll[3], t.group, t.nbr_flat, t.nbr_wide);
+                                t.unroll[2], t.unroll[3], t.group, 0u, t.nbr_wide);
   if (len <= 0 || len >= (int)sizeof line) return;
   // one short line written at once in append mode: lines of worlds tuned at
   // the same time by other processes do not interleave
@@ -2665,8 +2674,6 @@ pf_status World::tune() {
     }
     tune_.group = 0;
     if (const char* g = std::getenv("PFSIM_GROUP")) tune_.group = (uint32_t)std::atoi(g);
-    tune_.nbr_flat = 0;
-    if (const char* fl = std::getenv("PFSIM_NBR_FLAT")) tune_.nbr_flat = std::atoi(fl) ? 1u : 0u;
     tune_.nbr_wide = 0;
     if (const char* nw = std::getenv("PFSIM_NBR_WIDE")) tune_.nbr_wide = std::atoi(nw) ? 1u : 0u;
     apply_grouping();
@@ -2719,14 +2726,12 @@ pf_status World::tune_trials() {
   for (int kind = 0; kind < 4; ++kind) {
     if (kind == kSlotVel && !vel) continue;
     float best = 1e30f;
-    uint32_t bb = 256, bu = 4, bf = 0;
-    for (uint32_t flat = 0; flat < (kind == kSlotNbr ? 2u : 1u); ++flat)
+    uint32_t bb = 256, bu = 4;
     for (uint32_t b : blocks)
       for (uint32_t u : unrolls) {
         if (u == 8 && b == 512) continue;
         tune_.block[kind] = b;
         tune_.unroll[kind] = u;
-        if (kind == kSlotNbr) tune_.nbr_flat = flat;
         float t = 0;
         PF_TRY(timed(
             [&] {
@@ -2740,12 +2745,10 @@ pf_status World::tune_trials() {
           best = t;
           bb = b;
           bu = u;
-          bf = kind == kSlotNbr ? tune_.nbr_flat : 0u;
         }
       }
     tune_.block[kind] = bb;
     tune_.unroll[kind] = bu;
-    if (kind == kSlotNbr) tune_.nbr_flat = bf;
     const uint32_t reps = kind == kSlotDelta ? iters : (kind == kSlotLambda ? iters - (fuse_dens_ ? 1u : 0u) : 1u);
     slot_total += best * reps;
   }

@@ -489,8 +489,6 @@ class World {
     // that only hold one fluid of one mass run their whole substep group by
     // group, so a group's lists and records stay in L2 across its passes
     uint32_t group = 0;
-    // the list build walks its nine rows as one sequence (k_s_neighbors kFlat)
-    uint32_t nbr_flat = 0;
     // list entries as whole 32-bit slots in every warp instead of 16-bit
     // offsets where they fit: fewer bytes against fewer decode instructions
     uint32_t nbr_wide = 0;
@@ -523,6 +521,8 @@ class World {
   void launch_tiles_build(const WorldView& V, uint32_t s);
   template <typename K, typename... A>
   void launch_fluid(uint32_t block, K kernel, const WorldView& V, A... args);
+  template <typename K, typename... A>
+  void launch_fluid_smem(uint32_t block, size_t smem, K kernel, const WorldView& V, A... args);
   uint32_t mem_lanes_ = 32;  // lanes per cluster member in the shape-matching gather
   void run_fluid_neighbors(const WorldView& V, uint32_t s);
   void run_fluid_lambda_delta(const WorldView& V, uint32_t r, uint32_t s, uint32_t it);

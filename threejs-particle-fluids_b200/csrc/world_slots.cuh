@@ -228,21 +228,32 @@ __device__ __forceinline__ void lambda_terms(const DevFluid& F, f3 xi, float4 xj
 // density and lambda of its first solver iteration from the same hits, in
 // the same order (nothing moves between the list and that pass when the
 // world has no surface impulses and no late drag and lift).
-// kFlat: the nine rows are walked as one sequence, kNbrUnroll candidates
-// per round across row ends, so a warp waits for its longest walk rather
-// than, row by row, for each row's longest (the same candidates in the same
-// order; the autotuner picks the faster form).
-template <uint32_t kNbrUnroll, bool kDens, bool kFlat>
-__global__ void k_s_neighbors(WorldView V, uint32_t sub) {
+//
+// About 165 candidates are tested per particle (a warp's longest rows make it
+// 216 rounds) for 33 hits, so the pass is bound by the instructions of a
+// test. A hit therefore goes to the lane's own column of shared memory as a
+// 16-bit offset (one store and one pointer step, under the test's predicate;
+// neighbouring lanes share a bank's word at most), and the list leaves from
+// there afterwards, eight entries of a lane as one 16-byte store: written
+// hit by hit to the list itself, addresses and scattered 2-byte stores cost
+// as much as the tests. The density reads its neighbours' slots from the
+// column as well. The gathers still want a large L1: at 3.6 M fluid
+// particles a pass took 1,328 us before, and with the columns 1,398, 1,211
+// and 1,269 us at 36, 45 and 58 % of the SM's memory for them (blocks in
+// flight against L1); 64 registers rather than the 82 it would take.
+// A warp whose rows reach over more than 65,536 slots stores whole slots,
+// straight to its list.
+constexpr uint32_t kHitBytes = kMaxNbr * 2;  // shared memory per thread of the list build
+template <uint32_t kNbrUnroll, bool kDens>
+__global__ void __maxnreg__(kNbrUnroll == 8 ? 128 : 64) k_s_neighbors(WorldView V, uint32_t sub) {
   pdl_begin();
+  extern __shared__ uint16_t s_hits[];
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_fchunk * kSegAlign) return;     // whole warps
   const uint32_t k = chunk_slot(V.fchunk, g);  // slots of the scenes with a fluid
   const DevScene& S = scene_at(V, k);
   if (sub >= S.substeps) return;               // whole chunks
   const uint32_t f = tag_fluid(V.cur.tag[k]);
-  // every lane of the warp takes part in choosing the list width; lanes of
-  // other materials (f == 0) leave after that
   const DevFluid& F = V.fluids[f ? f - 1 : 0];
   const float4 xi4 = V.cur.xs[k];
   const f3 xi = xyz(xi4);
@@ -250,6 +261,11 @@ __global__ void k_s_neighbors(WorldView V, uint32_t sub) {
   float rho = 0.0f, gss = 0.0f;
   f3 gs = mk(0.0f, 0.0f, 0.0f);
   const float* __restrict__ q_of = reinterpret_cast<const float*>(V.lm) + 1;
+  const float qh = -S.homog_mass;
+  const bool homog = S.homog;
+  // a neighbour's record and terms for that density
+  auto fetch = [&](uint32_t j) { return NbrXQ{__ldg(V.cur.xs + j), homog ? qh : __ldg(q_of + 2 * (size_t)j)}; };
+  auto use = [&](uint32_t, const NbrXQ& r) { lambda_terms(F, xi, r.x, r.q, rho, gs, gss); };
   const float hsq = F.hsq;
   int32_t cx, cy, cz;
   local_cell(S, xi, &cx, &cy, &cz, nullptr);
@@ -290,137 +306,129 @@ __global__ void k_s_neighbors(WorldView V, uint32_t sub) {
     rs[r] = __ldg(V.cstart + row + a0);
     re[r] = __ldg(V.cstart + row + a1) + __ldg(V.ccount + row + a1);
   }
-  // The warp's entries are 16-bit offsets from the lowest slot its rows
-  // reach when every reachable slot lies within 65,536 of it.
-  // (No reduction when the world keeps whole slots in every warp.)
-  bool narrow = false;
-  uint32_t base = kNbrWide;
-  if (!V.nbr_wide_only) {  // uniform over the launch
-    uint32_t lo = 0xffffffffu, hi = 0;
+  // every lane takes part in the warp's reach; then lanes of other materials
+  // (f == 0) leave
+  uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll
-    for (int r = 0; r < 9; ++r) {
-      if (!f) rs[r] = re[r] = 0;
-      if (re[r] > rs[r]) {
-        lo = min(lo, rs[r]);
-        hi = max(hi, re[r]);
-      }
+  for (int r = 0; r < 9; ++r) {
+    if (!f) rs[r] = re[r] = 0;
+    if (re[r] > rs[r]) {
+      lo = min(lo, rs[r]);
+      hi = max(hi, re[r]);
     }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    narrow = hi <= lo || hi - lo <= 65536u;
-    base = narrow ? (hi > lo ? lo : 0u) : kNbrWide;
   }
-  if ((threadIdx.x & 31u) == 0) V.nbr_base[k >> 5] = base;
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  const bool staged = hi <= lo || hi - lo <= 65536u;
+  // the width of the list's entries (uniform over the warp)
+  const bool narrow = staged && !V.nbr_wide_only;
+  if ((threadIdx.x & 31u) == 0) V.nbr_base[k >> 5] = narrow ? (hi > lo ? lo : 0u) : kNbrWide;
   if (!f) return;
   // Every candidate is tested; the first kMaxNbr hits in walk order are
   // stored (as the reference's list keeps them) and any further hit only
-  // marks the overflow. The walk is compiled once per entry width (the width
-  // is uniform over the warp), and a 16-bit entry is stored without a branch
-  // on the count: hits past the kMaxNbr-th land in the group after the last,
-  // which the 16-bit layout leaves unused (a block has room for 2 kMaxNbr
-  // entries per slot).
+  // marks the overflow.
   uint32_t cnt = 0;
   uint32_t* __restrict__ out = V.nbr + nbr_col(k);
-  uint16_t* __restrict__ out16 = reinterpret_cast<uint16_t*>(V.nbr) + nbr16_col(k);
-  auto walk = [&](auto narrow_tag) {
-    constexpr bool kNarrow = decltype(narrow_tag)::value;
-    auto test = [&](uint32_t j, float4 xj) {
-      const bool hit = dist2_rn(xi, xj) < hsq;
-      if (kNarrow) {
-        if (hit)
-          out16[(min(cnt, kMaxNbr) / kNbrGroup) * (kNbrStride * kNbrGroup) + cnt % kNbrGroup] = (uint16_t)(j - base);
-      } else {
-        if (hit && cnt < kMaxNbr) out[cnt * kNbrStride] = j;
-      }
-      cnt += hit ? 1u : 0u;
-    };
-    if (kFlat) {
-      // the row pointer moves on at each row's end (empty rows skipped); the
-      // rows stay in registers (constant indices after unrolling)
-      int r = 0;
-      uint32_t j = rs[0], e = re[0];
-      auto pick = [](const uint32_t(&a)[9], int q) {
-        uint32_t v = a[0];
+  // whole rounds of a row, then its last 1 to kNbrUnroll - 1 candidates as one
+  // guarded round (a round's loads in flight together)
+  auto walk_row = [&](uint32_t j, uint32_t e, auto&& test) {
+    for (; j + kNbrUnroll <= e; j += kNbrUnroll) {
+      float4 xj[kNbrUnroll];
 #pragma unroll
-        for (int t = 1; t < 9; ++t) v = q == t ? a[t] : v;
-        return v;
-      };
-      auto advance = [&]() {
-        while (j >= e && r < 8) {
-          ++r;
-          j = pick(rs, r);
-          e = pick(re, r);
-        }
-      };
-      advance();
-      while (j < e) {
-        uint32_t c[kNbrUnroll];
-        bool live[kNbrUnroll];
+      for (uint32_t q = 0; q < kNbrUnroll; ++q) xj[q] = __ldg(V.cur.xs + j + q);
 #pragma unroll
-        for (uint32_t q = 0; q < kNbrUnroll; ++q) {
-          live[q] = j < e;
-          c[q] = j;
-          if (live[q]) {
-            ++j;
-            if (j >= e) advance();
-          }
-        }
-        float4 xj[kNbrUnroll];
+      for (uint32_t q = 0; q < kNbrUnroll; ++q) test(j + q, dist2_rn(xi, xj[q]) < hsq);
+    }
+    if (j < e) {
+      float4 xj[kNbrUnroll];
 #pragma unroll
-        for (uint32_t q = 0; q < kNbrUnroll; ++q)
-          if (live[q]) xj[q] = __ldg(V.cur.xs + c[q]);
+      for (uint32_t q = 0; q < kNbrUnroll; ++q)
+        if (j + q < e) xj[q] = __ldg(V.cur.xs + j + q);
 #pragma unroll
-        for (uint32_t q = 0; q < kNbrUnroll; ++q)
-          if (live[q]) test(c[q], xj[q]);
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < 9; ++r) {
-        uint32_t j = rs[r];
-        const uint32_t e = re[r];
-        // whole rounds, then the row's last 1 to kNbrUnroll - 1 candidates as
-        // one guarded round (their loads in flight together)
-        for (; j + kNbrUnroll <= e; j += kNbrUnroll) {
-          float4 xj[kNbrUnroll];
-#pragma unroll
-          for (uint32_t q = 0; q < kNbrUnroll; ++q) xj[q] = __ldg(V.cur.xs + j + q);
-#pragma unroll
-          for (uint32_t q = 0; q < kNbrUnroll; ++q) test(j + q, xj[q]);
-        }
-        if (j < e) {
-          float4 xj[kNbrUnroll];
-#pragma unroll
-          for (uint32_t q = 0; q < kNbrUnroll; ++q)
-            if (j + q < e) xj[q] = __ldg(V.cur.xs + j + q);
-#pragma unroll
-          for (uint32_t q = 0; q < kNbrUnroll; ++q)
-            if (j + q < e) test(j + q, xj[q]);
-        }
-      }
+      for (uint32_t q = 0; q < kNbrUnroll; ++q)
+        if (j + q < e) test(j + q, dist2_rn(xi, xj[q]) < hsq);
     }
   };
-  if (narrow)
-    walk(std::true_type{});
-  else
-    walk(std::false_type{});
+  uint16_t* const col = s_hits + (threadIdx.x / 32u) * (kMaxNbr * 32u) + (threadIdx.x & 31u);
+  if (staged) {
+    uint16_t* at = col;
+    uint16_t* const full = col + kMaxNbr * 32u;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      // whether every lane's candidates would fit, were they all hits (one
+      // decision for the warp, so that it walks the row once)
+      if (!__any_sync(__activemask(), at + (re[r] - rs[r]) * 32u > full)) {
+        walk_row(rs[r], re[r], [&](uint32_t j, bool hit) {
+          if (hit) {
+            *at = (uint16_t)(j - lo);
+            at += 32;
+          }
+        });
+      } else {
+        walk_row(rs[r], re[r], [&](uint32_t j, bool hit) {
+          if (!hit) return;
+          if (at < full) {
+            *at = (uint16_t)(j - lo);
+            at += 32;
+          } else {
+            ++cnt;  // past the kMaxNbr-th
+          }
+        });
+      }
+    }
+    cnt += (uint32_t)(at - col) / 32u;
+  } else {
+#pragma unroll
+    for (int r = 0; r < 9; ++r)
+      walk_row(rs[r], re[r], [&](uint32_t j, bool hit) {
+        if (hit && cnt < kMaxNbr) out[cnt * kNbrStride] = j;
+        cnt += hit ? 1u : 0u;
+      });
+  }
   const bool over = cnt > kMaxNbr;
   cnt = min(cnt, kMaxNbr);
   V.ncount[k] = cnt;
   if (over) atomicOr(V.flags + scene_index(V, k) * kNumFlags + FLAG_NBR, 1u);
-  if (kDens && dens) {
-    // the density pass over the list just written (still in cache), in list
-    // order, outside the divergent walk
-    NbrList L;
-    L.base = base;
-    L.w32 = V.nbr + nbr_col(k);
-    L.w16 = reinterpret_cast<const uint16_t*>(V.nbr) + nbr16_col(k);
-    const float qh = -S.homog_mass;
-    const bool homog = S.homog;
-    walk_nbrs<kNbrUnroll, true>(
-        L, cnt, [&](uint32_t j) { return NbrXQ{__ldg(V.cur.xs + j), homog ? qh : __ldg(q_of + 2 * (size_t)j)}; },
-        [&](uint32_t, const NbrXQ& r) { lambda_terms(F, xi, r.x, r.q, rho, gs, gss); });
-    finish_lambda(V, S, F, k, xi4, rho, gs, gss);
+  if (!staged) {
+    if (kDens && dens) {
+      NbrList L;
+      L.base = kNbrWide;
+      L.w32 = out;
+      L.w16 = nullptr;
+      walk_nbrs<kNbrUnroll, true>(L, cnt, fetch, use);
+      finish_lambda(V, S, F, k, xi4, rho, gs, gss);
+    }
+    return;
   }
+  // the column out, a group of kNbrGroup entries at a time (entries past cnt
+  // are whatever the column holds: no reader uses them), and the density over
+  // it, in list order
+  uint16_t* const out16 = reinterpret_cast<uint16_t*>(V.nbr) + nbr16_col(k);
+  for (uint32_t m = 0; m < cnt; m += kNbrGroup) {
+    uint32_t e[kNbrGroup];
+#pragma unroll
+    for (uint32_t q = 0; q < kNbrGroup; ++q) e[q] = col[(m + q) * 32u];
+    if (narrow) {
+      *reinterpret_cast<uint4*>(out16 + m * kNbrStride) =
+          make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+    } else {
+#pragma unroll
+      for (uint32_t q = 0; q < kNbrGroup; ++q) out[(m + q) * kNbrStride] = lo + e[q];
+    }
+    if (kDens && dens) {
+#pragma unroll
+      for (uint32_t q0 = 0; q0 < kNbrGroup; q0 += kNbrUnroll) {
+        NbrXQ rec[kNbrUnroll];
+#pragma unroll
+        for (uint32_t q = 0; q < kNbrUnroll; ++q)
+          if (m + q0 + q < cnt) rec[q] = fetch(lo + e[q0 + q]);
+#pragma unroll
+        for (uint32_t q = 0; q < kNbrUnroll; ++q)
+          if (m + q0 + q < cnt) use(0u, rec[q]);
+      }
+    }
+  }
+  if (kDens && dens) finish_lambda(V, S, F, k, xi4, rho, gs, gss);
 }
 
 // lambda.ts:41-71
