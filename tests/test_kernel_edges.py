@@ -127,3 +127,49 @@ def test_list_build_columns(oracle, monkeypatch, per_cell, unroll, wide):
     # densities: sums of at most 64 positive terms, each rounded a few times
     np.testing.assert_allclose(a.readback(N.PF_FIELD_DENSITY), b.readback(N.PF_FIELD_DENSITY), rtol=2e-5)
     a.close()
+
+
+@pytest.mark.parametrize("case", ["one", "overflow", "two_fluids", "boundary"])
+@pytest.mark.parametrize("unroll", [2, 4, 8])
+def test_surface_impulses_gathered_or_scattered(oracle, monkeypatch, case, unroll):
+    """Surface tension and adhesion where every particle gathers its own
+    changes (one fluid, with and without boundary particles) and where pairs
+    are scattered (an overflowing list; two fluids): the oracle's positions
+    and velocities."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    monkeypatch.setenv("PFSIM_NBR_PATH", "0")
+    monkeypatch.setenv("PFSIM_SLOT_BLOCK", "128")
+    monkeypatch.setenv("PFSIM_SLOT_UNROLL", str(unroll))
+    s = 0.02
+    g = np.stack(np.meshgrid(*[np.arange(9)] * 3, indexing="ij"), -1).reshape(-1, 3) * s
+    r = np.random.default_rng(unroll)
+    pos = (0.3 + g + r.uniform(-0.1 * s, 0.1 * s, g.shape)).astype(np.float32)
+    if case == "overflow":  # 90 particles in one cell's reach
+        pos[:90] = (0.3 + r.uniform(0, 0.6 * s, (90, 3))).astype(np.float32)
+    n, m = len(pos), len(pos) // 2
+    opts = dict(rest_density=1000.0, particle_spacing=s, smoothing_radius=2 * s, viscosity=0.01, surface_tension=0.1,
+                adhesion=0.1)
+    if case == "two_fluids":
+        mats = [("fluid", R.FluidOpts(range=(0, m), **opts)), ("fluid", R.FluidOpts(range=(m, n - m), **opts))]
+    elif case == "boundary":
+        mats = [("fluid", R.FluidOpts(range=(0, m), boundaries=[(m, n - m)], boundary_static=[True], **opts))]
+    else:
+        mats = [("fluid", R.FluidOpts(range=(0, n), **opts))]
+    w = None
+    if case == "boundary":
+        w = np.zeros(n, np.float32)
+    rec = R.Recipe(capacity=n, radius=s / 2, uploads=[R.Upload(0, pos, None, w)], materials=mats,
+                   loop=R.LoopOpts(substeps=2, iterations=2))
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    a.step(1 / 120)
+    b.step(1 / 120)
+    # (the oracle's flag is the last substep's list's, the scene's the frame's)
+    assert a.overflow()["neighbors"] == (case == "overflow")
+    x, y = a.readback(N.PF_FIELD_POSITIONS), b.readback(N.PF_FIELD_POSITIONS)
+    # 1e-5 of the block's 0.18 m would be 1.8e-6; the clump of `overflow`
+    # is pushed apart by metres per second, so its bound is relative to that
+    tol = 2e-6 if case != "overflow" else 1e-4 * max(1.0, float(np.abs(y).max()))
+    assert np.abs(x - y).max() <= tol
+    a.close()

@@ -2425,20 +2425,22 @@ void World::launch_fluid_smem(uint32_t block, size_t smem, K kernel, const World
       else launch_fluid_smem(b_, m_, k_s_neighbors<4, false>, __VA_ARGS__);             \
     }                                                                                   \
   } while (0)
-// XSPH, without the boundary-volume gather when the world has no boundaries.
-#define PF_XSPH(...)                                                                    \
+// A velocity-stage kernel at its tuned block size and fetch depth, without
+// the boundary-volume gather when the world has no boundaries.
+#define PF_BY_BND(K, ...)                                                               \
   do {                                                                                  \
     const uint32_t b_ = tune_.block[kSlotVel], u_ = tune_.unroll[kSlotVel];             \
     if (any_static_bnd_ || any_dyn_bnd_) {                                              \
-      if (u_ == 2) launch_fluid(b_, k_s_xsph<2, true>, __VA_ARGS__);                    \
-      else if (u_ == 8) launch_fluid(b_, k_s_xsph<8, true>, __VA_ARGS__);               \
-      else launch_fluid(b_, k_s_xsph<4, true>, __VA_ARGS__);                            \
+      if (u_ == 2) launch_fluid(b_, K<2, true>, __VA_ARGS__);                           \
+      else if (u_ == 8) launch_fluid(b_, K<8, true>, __VA_ARGS__);                      \
+      else launch_fluid(b_, K<4, true>, __VA_ARGS__);                                   \
     } else {                                                                            \
-      if (u_ == 2) launch_fluid(b_, k_s_xsph<2, false>, __VA_ARGS__);                   \
-      else if (u_ == 8) launch_fluid(b_, k_s_xsph<8, false>, __VA_ARGS__);              \
-      else launch_fluid(b_, k_s_xsph<4, false>, __VA_ARGS__);                           \
+      if (u_ == 2) launch_fluid(b_, K<2, false>, __VA_ARGS__);                          \
+      else if (u_ == 8) launch_fluid(b_, K<8, false>, __VA_ARGS__);                     \
+      else launch_fluid(b_, K<4, false>, __VA_ARGS__);                                  \
     }                                                                                   \
   } while (0)
+#define PF_XSPH(...) PF_BY_BND(k_s_xsph, __VA_ARGS__)
 // The position pass, without the boundary-reaction code when no fluid has
 // boundaries.
 #define PF_DELTA(...)                                                                   \
@@ -2918,8 +2920,8 @@ void World::run_substep(uint32_t s, uint32_t parity) {
         imp = imp || (F.rank == r && (F.has_st || F.has_ad));
       }
       if (!imp) continue;
-      if (st) PF_BY_UNROLL(kSlotVel, k_s_color_normal, VF, r, s);
-      PF_BY_UNROLL(kSlotVel, k_s_impulses, VF, r, s);
+      if (st) PF_BY_BND(k_s_color_normal, VF, r, s);
+      PF_BY_BND(k_s_impulses, VF, r, s);
       launch_slots(k_imp_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s);
     }
   launch_aero(V, 1, s);
@@ -2995,7 +2997,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
     for (auto& D : h_softs_) has_local = has_local || (D.rank == r && D.local);
     if (has_velocity && VF.n_fchunk) {
       run_fluid_xsph(VF, r, s);
-      if (has_vort) PF_BY_UNROLL(kSlotVel, k_s_vort_grad, VF, r, s);
+      if (has_vort) PF_BY_BND(k_s_vort_grad, VF, r, s);
       launch_slots(k_xsph_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s);
     }
     if (has_local) {
