@@ -173,3 +173,24 @@ def test_surface_impulses_gathered_or_scattered(oracle, monkeypatch, case, unrol
     tol = 2e-6 if case != "overflow" else 1e-4 * max(1.0, float(np.abs(y).max()))
     assert np.abs(x - y).max() <= tol
     a.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 1_023, 16_384, 16_385, 32_769, 65_536, 65_537])
+@pytest.mark.parametrize("dims", [(2, 1, 1), (16, 16, 1), (17, 16, 1), (64, 64, 64), (64, 64, 65), (200, 100, 100)])
+def test_sort_in_one_cluster(oracle, n, dims):
+    """The sort of few elements in one thread-block cluster and its limits:
+    one to four elements a thread, one to three passes, cell counts scanned in
+    the cluster or after it; spread over the grid, and half of them in one
+    cell. The oracle's keys, counts, starts and permutation."""
+    from pfsim import hashgrid as H
+
+    r = np.random.default_rng(n + dims[0])
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, :3] = r.uniform(0.0, 1.0, (n, 3)) * np.array(dims) * 0.1
+    pos[: n // 2, :3] = pos[n - 1, :3]
+    g = H.GridOptions(cell_size=0.1, kind="linear", dims=dims)
+    a, b = H.sort(pos, g), oracle.sort(pos, g.desc(n))
+    assert np.array_equal(a.cell_index, b["keys"])
+    assert np.array_equal(a.counts, b["count"])
+    assert np.array_equal(a.cell_start, b["start"])
+    assert np.array_equal(a.sorted_indices, b["perm"])

@@ -99,24 +99,40 @@ class LinkedLaunches {
 // plainly, after all of the stream's work before it.
 inline void break_link() { t_link.linked = false; }
 
-// kernel<<<grid, block, smem, st>>>(args...), linked where the operation
-// before it on this thread was a kernel on the same stream. Every kernel
-// launched through it starts with pdl_begin().
-template <typename... P, typename... A>
-inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline cudaLaunchAttribute cluster_attribute(uint32_t blocks) {
   cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  return at;
+}
+// kernel<<<grid, block, smem, st>>>(args...) in clusters of `cluster` blocks
+// (0: none), linked where the operation before it on this thread was a kernel
+// on the same stream. Every kernel launched through it starts with pdl_begin().
+template <typename... P, typename... A>
+inline cudaError_t launch_cluster(void (*kernel)(P...), uint32_t cluster, dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t st, A... args) {
+  cudaLaunchAttribute at[2] = {};
+  unsigned attrs = 0;
+  if (t_link.on && t_link.linked && t_link.last == st) {
+    at[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[attrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster) at[attrs++] = cluster_attribute(cluster);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cfg.attrs = &at;
-  cfg.numAttrs = t_link.on && t_link.linked && t_link.last == st ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = attrs;
   t_link.linked = true;
   t_link.last = st;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  return launch_cluster(kernel, 0, grid, block, smem, st, args...);
 }
 
 __host__ __device__ inline uint32_t div_up(uint32_t a, uint32_t b) { return (a + b - 1) / b; }

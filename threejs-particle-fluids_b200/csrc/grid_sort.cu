@@ -264,11 +264,14 @@ k_keys_digits(const float4* pos, uint32_t n, KeyFn kf, DigitHist h, uint32_t* ke
 
 // Each pass's digit counts -> each digit's first output position (one block
 // of 1024 threads per pass, two digits per thread).
-__global__ void __launch_bounds__(1024) k_digit_first(uint32_t* __restrict__ dc, uint32_t digits) {
+// `over_to`, unless NULL, receives the keys' overflow flag.
+__global__ void __launch_bounds__(1024) k_digit_first(uint32_t* dc, uint32_t digits, const uint32_t* over,
+                                                      uint32_t* over_to) {
   pdl_begin();
   __shared__ uint32_t s_warp[32];
   uint32_t* c = dc + blockIdx.x * kRadixMaxDigits;
   const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
+  if (over_to && blockIdx.x == 0 && t == 0) *over_to = *over;
   const uint32_t a = 2 * t < digits ? c[2 * t] : 0u, b = 2 * t + 1 < digits ? c[2 * t + 1] : 0u;
   const uint32_t own = a + b;
   uint32_t x = own;
@@ -613,6 +616,203 @@ k_radix_scatter(const uint32_t* kin, const uint32_t* vin, uint32_t n, uint32_t* 
   }
 }
 
+// ------------------------------------------------------------ small sort ----
+// A sort of at most 65,536 elements in one thread-block cluster: every
+// pass, and the scan of the cell counts where the cells are few, in one
+// launch. A pass of the kernels above is three or four launches of a few
+// microseconds each, however few the elements; here the blocks exchange their
+// digit counts through distributed shared memory and meet at the hardware
+// cluster barrier. The elements stay in registers within a pass and go from
+// pass to pass through L2. Ranks as in k_radix_scatter: by ballots within a
+// warp, against the warp's histogram over its rounds, over the block's warps,
+// then over the blocks, so the sort is stable.
+// A sort of 20,011 particles (two passes, 65,536 cells) took 40 us as linked
+// launches and takes 25 so; the sorts of a 50,000-particle pile's step (three
+// passes) went from about 45 to 29 us each. Above 65,536 elements more SMs
+// than a cluster's are worth the launches.
+constexpr uint32_t kSmallThreads = 1024;
+constexpr uint32_t kSmallWarps = kSmallThreads / 32;
+constexpr uint32_t kSmallItems = 4;      // elements per thread at most
+constexpr uint32_t kSmallBlocks = 16;    // blocks of the cluster (8 where 16 cannot be resident)
+constexpr uint32_t kSmallDigits = 256;   // passes of 8 bits at most
+constexpr uint64_t kSmallScan = 262144;  // cells scanned in the cluster at most (else k_scan follows)
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// Word `p` (a shared variable of every block) of block `rank`.
+__device__ __forceinline__ uint32_t cluster_load(const uint32_t* p, uint32_t rank) {
+  uint32_t a, v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// kItems elements per thread; passes of `width` bits, digits = 1 << width.
+// `a`, `b`: the passes' outputs in turn, as (key, element) pairs, which one
+// 8-byte store each scatters (the last pass writes perm). `over_to`, unless
+// NULL, receives the keys' overflow flag.
+template <uint32_t kItems>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, uint2* a, uint2* b, uint32_t* perm,
+             uint32_t* count, uint32_t* start, uint32_t cells, uint32_t scan, const uint32_t* over, uint32_t* over_to) {
+  pdl_begin();
+  __shared__ uint16_t whist[kSmallWarps][kSmallDigits];  // per warp: its digit counts, then their offsets
+  __shared__ uint32_t part[4][kSmallDigits], prior[4][kSmallDigits], whole[4][kSmallDigits];
+  __shared__ uint32_t mine[kSmallDigits];   // this block's digit counts (read by the others)
+  __shared__ uint32_t first[kSmallDigits];  // first output position of this block's elements of each digit
+  __shared__ uint32_t s_warp[kSmallWarps];
+  __shared__ uint32_t total;                // of this block's cells (read by the others)
+  uint32_t blocks, me;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(blocks));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(me));
+  const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, lt = lanemask_lt();
+  const uint32_t digits = 1u << width, mask = digits - 1u;
+  const uint32_t base = (me * kSmallWarps + warp) * (32u * kItems) + lane;  // element i of the thread: base + 32 i
+  const uint32_t d4 = tid & (kSmallDigits - 1u), quarter = tid / kSmallDigits;
+  // exclusive sum of v over the block's threads
+  auto block_exclusive = [&](uint32_t v, uint32_t* sum) {
+    uint32_t x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= (uint32_t)off) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    const uint32_t w = s_warp[lane];
+    uint32_t wi = w;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, wi, off);
+      if (lane >= (uint32_t)off) wi += y;
+    }
+    *sum = __shfl_sync(0xffffffffu, wi, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, wi - w, warp);
+    __syncthreads();  // s_warp is free again
+    return before + x - v;
+  };
+  if (over_to && me == 0 && tid == 0) *over_to = *over;
+  const uint2* in = nullptr;
+  for (uint32_t p = 0; p < passes; ++p) {
+    const uint32_t shift = p * width;
+    const bool last = p + 1 == passes;
+    uint32_t key[kItems], val[kItems], pos[kItems];
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; ++i) {
+      const uint32_t e = base + 32u * i;
+      key[i] = 0u;
+      val[i] = e;
+      if (e >= n) continue;
+      if (in) {
+        const uint2 kv = __ldcg(in + e);
+        key[i] = kv.x;
+        val[i] = kv.y;
+      } else {
+        key[i] = __ldcg(keys + e);
+      }
+    }
+    for (uint32_t w = lane; w < kSmallDigits / 2; w += 32) reinterpret_cast<uint32_t*>(whist[warp])[w] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; ++i) {
+      const bool ok = base + 32u * i < n;
+      const uint32_t live = __ballot_sync(0xffffffffu, ok);
+      pos[i] = 0;
+      if (!live) continue;  // warp-uniform
+      const uint32_t d = (key[i] >> shift) & mask;
+      uint32_t pm = 0, old = 0;
+      if (ok) {
+        pm = digit_peers<0>(d, width, live);
+        old = whist[warp][d];
+        pos[i] = old + __popc(pm & lt);
+        if (p == 0) {  // the cell counts: one atomic per key of the round
+          const uint32_t same = __match_any_sync(live, key[i]);
+          if (lane == (uint32_t)(__ffs(same) - 1)) atomicAdd(count + key[i], (uint32_t)__popc(same));
+        }
+      }
+      __syncwarp();
+      if (ok && lane == (uint32_t)(__ffs(pm) - 1)) whist[warp][d] = (uint16_t)(old + __popc(pm));
+      __syncwarp();
+    }
+    __syncthreads();
+    // per digit, eight warps to a thread: their counts -> offsets
+    {
+      uint32_t sum = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < kSmallWarps / 4; ++w) {
+        uint16_t* h = &whist[quarter * (kSmallWarps / 4) + w][d4];
+        const uint32_t c = *h;
+        *h = (uint16_t)sum;
+        sum += c;
+      }
+      part[quarter][d4] = sum;
+    }
+    __syncthreads();
+    if (tid < kSmallDigits) mine[tid] = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid];
+    cluster_sync();
+    // per digit: the blocks' counts in all, and those of the blocks before
+    {
+      uint32_t all = 0, before = 0;
+      for (uint32_t r = quarter; r < blocks; r += 4) {
+        const uint32_t c = cluster_load(mine + d4, r);
+        all += c;
+        before += r < me ? c : 0u;
+      }
+      static_assert(kSmallThreads == 4 * kSmallDigits, "four threads a digit");
+      prior[quarter][d4] = before;
+      whole[quarter][d4] = all;
+      __syncthreads();
+      uint32_t sum;
+      const uint32_t own = tid < kSmallDigits ? whole[0][tid] + whole[1][tid] + whole[2][tid] + whole[3][tid] : 0u;
+      const uint32_t excl = block_exclusive(own, &sum);
+      if (tid < kSmallDigits) first[tid] = excl + prior[0][tid] + prior[1][tid] + prior[2][tid] + prior[3][tid];
+    }
+    __syncthreads();
+    uint2* out = (p & 1u) ? b : a;
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; ++i)
+      if (base + 32u * i < n) {
+        const uint32_t d = (key[i] >> shift) & mask;
+        uint32_t dst = first[d] + whist[warp][d] + pos[i];
+        for (uint32_t q = 0; q < warp / (kSmallWarps / 4); ++q) dst += part[q][d];
+        if (last) perm[dst] = val[i];
+        else out[dst] = make_uint2(key[i], val[i]);
+      }
+    cluster_sync();
+    in = out;
+  }
+  if (!scan) return;
+  // cell counts -> starts: a run of cells per block, 4 a thread and round
+  const uint32_t per = (div_up(cells, blocks) + 3u) & ~3u;
+  const uint32_t c0 = min(me * per, cells), c1 = min(c0 + per, cells);
+  uint32_t sum = 0, block_sum;
+  for (uint32_t c = c0 + tid; c < c1; c += kSmallThreads) sum += __ldcg(count + c);
+  (void)block_exclusive(sum, &block_sum);
+  if (tid == 0) total = block_sum;
+  cluster_sync();
+  uint32_t carry = 0;
+  {
+    const uint32_t t = lane < blocks && lane < me ? cluster_load(&total, lane) : 0u;
+    carry = __reduce_add_sync(0xffffffffu, t);
+  }
+  for (uint32_t cc = c0; cc < c1; cc += 4u * kSmallThreads) {
+    const uint32_t c = cc + 4u * tid;
+    uint32_t v[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) v[q] = c + q < c1 ? __ldcg(count + c + q) : 0u;
+    uint32_t round;
+    uint32_t at = carry + block_exclusive(v[0] + v[1] + v[2] + v[3], &round);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      if (c + q < c1) start[c + q] = at;
+      at += v[q];
+    }
+    carry += round;
+  }
+  cluster_sync();  // no block leaves while another may read its total
+}
+
 // A plan of no passes (one cell): the identity permutation.
 __global__ void __launch_bounds__(256) k_identity(uint32_t* __restrict__ perm, uint32_t n) {
   pdl_begin();
@@ -780,8 +980,8 @@ cudaError_t sort_state_zero(const SortScratch& s, uint64_t C, cudaStream_t st) {
 
 void launch_keys_digits(const float4* pos, uint32_t n, const KeyFn& kf, const RadixPlan& plan, uint32_t* keys,
                         uint32_t* overflow, uint32_t* count, uint64_t C, const SortScratch& s, cudaStream_t st) {
-  const DigitHist h = digit_hist(plan, s);
-  launch_kernel(k_keys_digits, keys_grid(n, C, kHistThreads), kHistThreads, 4ull * plan.passes * plan.digits, st, pos, n, kf, h, keys,
+  const DigitHist h = digit_hist(plan, s, n);
+  launch_kernel(k_keys_digits, keys_grid(n, C, kHistThreads), kHistThreads, 4ull * h.passes * h.digits, st, pos, n, kf, h, keys,
                 overflow, count, C);
 }
 
@@ -861,8 +1061,57 @@ cudaError_t scatter_allow_smem_all() {
 }
 }  // namespace
 
-uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n) {
+namespace {
+// Per device (radix_prepare): blocks of k_small_sort's cluster, 0 where none
+// can be resident.
+uint32_t g_small_blocks[64];
+uint32_t small_blocks() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev < 64 ? g_small_blocks[dev] : 0u;
+}
+cudaLaunchConfig_t small_config(uint32_t blocks, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.stream = st;
+  return cfg;
+}
+template <uint32_t kItems>
+uint32_t small_blocks_of() {
+  if (cudaFuncSetAttribute(k_small_sort<kItems>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return 8;
+  cudaLaunchAttribute at = cluster_attribute(kSmallBlocks);
+  cudaLaunchConfig_t cfg = small_config(kSmallBlocks, nullptr);
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  return cudaOccupancyMaxActiveClusters(&clusters, k_small_sort<kItems>, &cfg) == cudaSuccess && clusters > 0
+             ? kSmallBlocks
+             : 8u;
+}
+cudaError_t launch_small_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan, uint32_t* count,
+                              uint32_t* start, uint32_t* perm, uint32_t* overflow, const SortScratch& s,
+                              cudaStream_t st) {
+  const uint32_t blocks = small_blocks(), lanes = blocks * kSmallThreads, scan = C <= kSmallScan ? 1u : 0u;
+  auto go = [&](auto kernel) {
+    // the scratch holds va behind ka (vb behind kb): room for n pairs
+    return launch_cluster(kernel, blocks, blocks, kSmallThreads, 0, st, keys, n, plan.passes, plan.width,
+                          reinterpret_cast<uint2*>(s.ka), reinterpret_cast<uint2*>(s.kb), perm, count, start,
+                          (uint32_t)C, scan, s.counters + kCounterOverflow, overflow);
+  };
+  if (n <= lanes) return go(k_small_sort<1>);
+  if (n <= 2 * lanes) return go(k_small_sort<2>);
+  return go(k_small_sort<kSmallItems>);
+}
+}  // namespace
+
+bool small_sort(const RadixPlan& plan, uint32_t n) {
+  return n > 0 && plan.passes > 0 && plan.digits <= kSmallDigits && n <= small_blocks() * kSmallThreads * kSmallItems;
+}
+
+uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n, uint64_t C) {
   if (n == 0) return 1;                        // the start scan
+  if (small_sort(plan, n)) return C <= kSmallScan ? 1u : 2u;
   if (plan.passes == 0) return 3;              // identity, run counts, start scan
   // digit scan, per pass four (three when the tiles form one chunk), start scan
   const uint32_t per_pass = div_up(radix_tiles(n), kScanChunk) > 1 ? 4u : 3u;
@@ -870,8 +1119,14 @@ uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n) {
 }
 
 cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan, uint32_t* count,
-                             uint32_t* start, uint32_t* perm, const SortScratch& s, cudaStream_t st) {
+                             uint32_t* start, uint32_t* perm, uint32_t* overflow, const SortScratch& s,
+                             cudaStream_t st) {
   if (C == 0) return cudaSuccess;
+  if (small_sort(plan, n)) {
+    if (cudaError_t e = launch_small_sort(keys, n, C, plan, count, start, perm, overflow, s, st); e != cudaSuccess)
+      return e;
+    return C <= kSmallScan ? cudaSuccess : launch_start_scan(count, start, C, s, st);
+  }
   if (n > 0) {
     const uint32_t tiles = radix_tiles(n);
     if (plan.passes == 0) {
@@ -879,7 +1134,8 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
       launch_kernel(k_run_counts, div_up(n, 256), 256, 0, st, keys, n, count);
     } else {
       if (cudaError_t e = radix_prepare(); e != cudaSuccess) return e;
-      launch_kernel(k_digit_first, plan.passes, 1024, 0, st, s.digit_count, plan.digits);
+      launch_kernel(k_digit_first, plan.passes, 1024, 0, st, s.digit_count, plan.digits,
+                    s.counters + kCounterOverflow, overflow);
       const uint32_t chunks = div_up(tiles, kScanChunk);
       const bool kvec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
       const uint32_t* kin = keys;
@@ -931,6 +1187,9 @@ cudaError_t radix_prepare() {
       e != cudaSuccess)
     return e;
   if (dev < 64) g_smem_per_sm[dev] = per_sm;
+  if (dev < 64)
+    g_small_blocks[dev] = std::min({small_blocks_of<1>(), small_blocks_of<2>(), small_blocks_of<kSmallItems>()});
+  cudaGetLastError();
   (void)sm_count();  // cached outside any stream capture
   ready.insert(dev);
   return cudaSuccess;
@@ -939,13 +1198,18 @@ cudaError_t radix_prepare() {
 cudaError_t sort_run(const float4* pos, uint32_t n, const KeyFn& kf, uint64_t C, uint32_t* perm, uint32_t* start,
                      uint32_t* count, uint32_t* keys, uint32_t* overflow, const SortScratch& s, cudaStream_t st) {
   const RadixPlan plan = radix_plan(C);
+  if (cudaError_t e = radix_prepare(); e != cudaSuccess) return e;
   LinkedLaunches scope;
   if (cudaError_t e = sort_state_zero(s, C, st); e != cudaSuccess) return e;
-  uint32_t* ovf = overflow ? overflow : s.counters + kCounterOverflow;
-  if (overflow)
+  // the flag is raised in the counters and copied out by the sort's kernels;
+  // without elements or passes, none of those runs
+  uint32_t* ovf = s.counters + kCounterOverflow;
+  if (overflow && (n == 0 || plan.passes == 0)) {
     if (cudaError_t e = cudaMemsetAsync(overflow, 0, 4, st); e != cudaSuccess) return e;
+    ovf = overflow;
+  }
   launch_keys_digits(pos, n, kf, plan, keys, ovf, count, C, s, st);
-  return launch_grid_sort(keys, n, C, plan, count, start, perm, s, st);
+  return launch_grid_sort(keys, n, C, plan, count, start, perm, overflow, s, st);
 }
 
 }  // namespace pf

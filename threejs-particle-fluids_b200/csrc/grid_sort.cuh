@@ -100,13 +100,16 @@ void launch_keys_digits(const float4* pos, uint32_t n, const KeyFn& kf, const Ra
 
 // The sort proper from keys by element (keys[e] < C) whose digit counts are
 // in s.digit_count: writes perm[n], count[C] (zeroed by the key kernel) and
-// start[C], after sort_state_zero.
+// start[C], after sort_state_zero. `overflow`, unless NULL, receives the flag
+// that the keys raised in the counters (plans of one pass or more).
 cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan,
-                             uint32_t* count, uint32_t* start, uint32_t* perm, const SortScratch& s,
-                             cudaStream_t st);
+                             uint32_t* count, uint32_t* start, uint32_t* perm, uint32_t* overflow,
+                             const SortScratch& s, cudaStream_t st);
 
-// Kernel launches of launch_grid_sort for a plan and element count.
-uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n);
+// Kernel launches of launch_grid_sort for a plan, element and cell count.
+uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n, uint64_t C);
+// Whether n elements are sorted in one cluster (after radix_prepare).
+bool small_sort(const RadixPlan& plan, uint32_t n);
 
 // Per device, once: the radix passes' shared-memory size above the default
 // limit. Call it outside stream capture before the first sort on a device
@@ -146,8 +149,10 @@ __device__ __forceinline__ void zero_counts(uint32_t* count, uint64_t cells) {
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += (uint64_t)gridDim.x * blockDim.x)
     count[c] = 0u;
 }
-inline DigitHist digit_hist(const RadixPlan& p, const SortScratch& s) {
-  return DigitHist{p.passes, p.width, p.digits, s.digit_count};
+// The digit counts that a sort of n elements starts from (none for one in a
+// cluster: it counts for itself).
+inline DigitHist digit_hist(const RadixPlan& p, const SortScratch& s, uint32_t n) {
+  return DigitHist{small_sort(p, n) ? 0u : p.passes, p.width, p.digits, s.digit_count};
 }
 // Blocks of a grid-stride key kernel over n elements that zeroes `cells`
 // counts: enough to fill the GPU, few enough that each block's histogram
