@@ -679,6 +679,8 @@ __global__ void __launch_bounds__(kBlock) k_damp_apply(WorldView V, uint32_t beg
 }
 
 // ---------------------------------------------------------- soft bodies ----
+constexpr uint32_t kSmBlock = 128;  // threads per block of the moment pass
+
 // A multiplier of the iteration before; zero in a substep's first iteration,
 // where every multiplier starts again (buildImplicitResetPairLambdaKernel),
 // so that nothing clears them in between.
@@ -758,62 +760,137 @@ __global__ void __launch_bounds__(kBlock) k_rot_advect(WorldView V, uint32_t sub
   V.q[i] = qp;
 }
 
+// The members' slots of this substep, for the moment passes of its iterations.
+__global__ void __launch_bounds__(kBlock) k_sm_slots(WorldView V) {
+  pdl_begin();
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < V.n_sm) V.sm_slots[e] = V.inv[V.sm_ids[e]];
+}
+
 // shapeMatchImplicit.ts:46-71 (the cluster's centre) and 100-217 (its moment
 // matrix and rotation), one thread per cluster. The moment of a cluster reads
 // only its own centre, so the thread forms the centre first, in CSR order as
 // the reference's centre pass does, and keeps it in registers; the members'
 // positions come back from cache for the moment.
-__global__ void __launch_bounds__(kBlock) k_sm_moment(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+//
+// Bound by the latency of the members' loads: a member's slot and id come
+// from lists laid out warp by warp (entry m of a warp's clusters is one line;
+// the slots are looked up once per substep), so that a member costs one
+// dependent load after a coalesced one, and eight (four in the moment)
+// members are in flight at a time, summed in CSR order. MOMENTTIMES
+__global__ void __launch_bounds__(kSmBlock) k_sm_moment(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
   pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
+  const uint4 G = V.sm_grp[g];  // id, first entry, members, entry stride
+  const uint32_t i = G.x, deg = G.z, stride = G.w;
+  const float4 rest_i = V.rest[i], cb4 = V.rest_c[i];
   const DevSoft* D;
   const DevScene* S;
   if (!group_active(V, g, rank, sub, it, &D, &S)) return;
-  const uint32_t i = V.grp[g];
-  const uint32_t s = V.csr_off[i], e = V.csr_off[i + 1];
+  const uint32_t* slots = V.sm_slots + G.y;
+  const uint32_t* ids = V.sm_ids + G.y;
   f3 sum = mk(0.0f, 0.0f, 0.0f);
-  for (uint32_t m = s; m < e; ++m) sum = sum + xyz(V.cur.xs[V.inv[V.csr_idx[m]]]);
-  const float inv_cnt = 1.0f / (float)max(e - s, 1u);
-  const f3 c = e == s ? mk(0.0f, 0.0f, 0.0f) : sum * inv_cnt;
+  for (uint32_t m = 0; m < deg; m += 8) {
+    float4 x[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q)
+      if (m + q < deg) x[q] = V.cur.xs[slots[(size_t)(m + q) * stride]];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q)
+      if (m + q < deg) sum = sum + xyz(x[q]);
+  }
+  const float inv_cnt = 1.0f / (float)max(deg, 1u);
+  const f3 c = deg == 0 ? mk(0.0f, 0.0f, 0.0f) : sum * inv_cnt;
   float a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  const f3 cb = xyz(V.rest_c[i]);
+  const f3 cb = xyz(cb4);
   const float ai = D->ai;
-  for (uint32_t m = s; m < e; ++m) {
-    const uint32_t j = V.csr_idx[m];
-    const float4 qj = V.qp[j];
-    const float xx = qj.x * qj.x, yy = qj.y * qj.y, zz = qj.z * qj.z, xy = qj.x * qj.y, xz = qj.x * qj.z,
-                yz = qj.y * qj.z, wx = qj.w * qj.x, wy = qj.w * qj.y, wz = qj.w * qj.z;
-    a[0] += ai * (1.0f - (yy + zz) * 2.0f);
-    a[1] += ai * ((xy - wz) * 2.0f);
-    a[2] += ai * ((xz + wy) * 2.0f);
-    a[3] += ai * ((xy + wz) * 2.0f);
-    a[4] += ai * (1.0f - (xx + zz) * 2.0f);
-    a[5] += ai * ((yz - wx) * 2.0f);
-    a[6] += ai * ((xz - wy) * 2.0f);
-    a[7] += ai * ((yz + wx) * 2.0f);
-    a[8] += ai * (1.0f - (xx + yy) * 2.0f);
-    const f3 xj = xyz(V.cur.xs[V.inv[j]]) - c;
-    const f3 xt = xyz(V.rest[j]) - cb;
-    a[0] += xj.x * xt.x;
-    a[1] += xj.x * xt.y;
-    a[2] += xj.x * xt.z;
-    a[3] += xj.y * xt.x;
-    a[4] += xj.y * xt.y;
-    a[5] += xj.y * xt.z;
-    a[6] += xj.z * xt.x;
-    a[7] += xj.z * xt.y;
-    a[8] += xj.z * xt.z;
+  for (uint32_t m = 0; m < deg; m += 4) {
+    float4 x[4], qn[4], rest[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      if (m + q < deg) {
+        const uint32_t j = ids[(size_t)(m + q) * stride];
+        x[q] = V.cur.xs[slots[(size_t)(m + q) * stride]];
+        qn[q] = V.qp[j];
+        rest[q] = V.rest[j];
+      }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      if (m + q >= deg) continue;
+      const float4 qj = qn[q];
+      const float xx = qj.x * qj.x, yy = qj.y * qj.y, zz = qj.z * qj.z, xy = qj.x * qj.y, xz = qj.x * qj.z,
+                  yz = qj.y * qj.z, wx = qj.w * qj.x, wy = qj.w * qj.y, wz = qj.w * qj.z;
+      a[0] += ai * (1.0f - (yy + zz) * 2.0f);
+      a[1] += ai * ((xy - wz) * 2.0f);
+      a[2] += ai * ((xz + wy) * 2.0f);
+      a[3] += ai * ((xy + wz) * 2.0f);
+      a[4] += ai * (1.0f - (xx + zz) * 2.0f);
+      a[5] += ai * ((yz - wx) * 2.0f);
+      a[6] += ai * ((xz - wy) * 2.0f);
+      a[7] += ai * ((yz + wx) * 2.0f);
+      a[8] += ai * (1.0f - (xx + yy) * 2.0f);
+      const f3 xj = xyz(x[q]) - c;
+      const f3 xt = xyz(rest[q]) - cb;
+      a[0] += xj.x * xt.x;
+      a[1] += xj.x * xt.y;
+      a[2] += xj.x * xt.z;
+      a[3] += xj.y * xt.x;
+      a[4] += xj.y * xt.y;
+      a[5] += xj.y * xt.z;
+      a[6] += xj.z * xt.x;
+      a[7] += xj.z * xt.y;
+      a[8] += xj.z * xt.z;
+    }
   }
   float r[9];
   polar3(a, r);
-  if (e == s) {
+  if (deg == 0) {
     r[0] = 1; r[1] = 0; r[2] = 0; r[3] = 0; r[4] = 1; r[5] = 0; r[6] = 0; r[7] = 0; r[8] = 1;
   }
   V.rot4[4 * (size_t)i + 0] = make_float4(r[0], r[1], r[2], c.x);
   V.rot4[4 * (size_t)i + 1] = make_float4(r[3], r[4], r[5], c.y);
   V.rot4[4 * (size_t)i + 2] = make_float4(r[6], r[7], r[8], c.z);
-  V.rot4[4 * (size_t)i + 3] = make_float4(cb.x, cb.y, cb.z, V.rest[i].w);
+  V.rot4[4 * (size_t)i + 3] = make_float4(cb.x, cb.y, cb.z, rest_i.w);
+}
+
+// shapeMatchImplicit.ts:325-401: the quaternion of cluster i's rotation, on the
+// side of its committed one.
+__device__ __forceinline__ void cluster_quaternion(const WorldView& V, uint32_t i) {
+  const float4 r0 = V.rot4[4 * (size_t)i], r1 = V.rot4[4 * (size_t)i + 1], r2 = V.rot4[4 * (size_t)i + 2];
+  const float m00 = r0.x, m01 = r0.y, m02 = r0.z, m10 = r1.x, m11 = r1.y, m12 = r1.z, m20 = r2.x, m21 = r2.y,
+              m22 = r2.z;
+  const float tr = m00 + m11 + m22;
+  float qx, qy, qz, qw;
+  if (tr > 0.0f) {
+    const float sq = 0.5f / sqrtf(tr + 1.0f);
+    qw = 0.25f / sq;
+    qx = (m21 - m12) * sq;
+    qy = (m02 - m20) * sq;
+    qz = (m10 - m01) * sq;
+  } else if (m00 > m11 && m00 > m22) {
+    const float sq = 2.0f * sqrtf(1.0f + m00 - m11 - m22);
+    qw = (m21 - m12) / sq;
+    qx = 0.25f * sq;
+    qy = (m01 + m10) / sq;
+    qz = (m02 + m20) / sq;
+  } else if (m11 > m22) {
+    const float sq = 2.0f * sqrtf(1.0f + m11 - m00 - m22);
+    qw = (m02 - m20) / sq;
+    qx = (m01 + m10) / sq;
+    qy = 0.25f * sq;
+    qz = (m12 + m21) / sq;
+  } else {
+    const float sq = 2.0f * sqrtf(1.0f + m22 - m00 - m11);
+    qw = (m10 - m01) / sq;
+    qx = (m02 + m20) / sq;
+    qy = (m12 + m21) / sq;
+    qz = 0.25f * sq;
+  }
+  const float4 q0 = V.q[i];
+  const float d = q0.x * qx + q0.y * qy + q0.z * qz + q0.w * qw;
+  const float fl = d < 0.0f ? -1.0f : 1.0f;
+  V.qp[i] = make_float4(qx * fl, qy * fl, qz * fl, qw * fl);
 }
 
 // shapeMatchImplicit.ts:248-308 taken by member, with the accumulator's
@@ -824,8 +901,9 @@ __global__ void __launch_bounds__(kBlock) k_sm_moment(WorldView V, uint32_t rank
 // warp, L chosen per world from how many clusters hold a particle): each lane
 // forms the corrections of clusters that hold it, term for term as the
 // cluster would, and updates those pairs' multipliers (each pair belongs to
-// one member); the lanes' tick sums are added across the group, and its first
-// lane applies them to the particle's predicted position. No other group
+// one member, and lies beside the member's others); the lanes' tick sums are
+// added across the group, and its first lane applies them to the particle's
+// predicted position. No other group
 // reads that position in this pass: the clusters' centres and rotations come
 // from the passes before. Every lane of a warp reaches the shuffles: a lane
 // past the last member, or whose member's body skips this pass, adds zero.
@@ -865,9 +943,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
     const float mj = fmaxf((float)(c1 - c0), 1.0f);
     const float dt2 = S->dt * S->dt;
     const float maxc2 = D->maxc2, scale = S->sb_scale;
+    const bool keep = it + 1 < S->iterations;  // the multipliers are read once more
     for (uint32_t q = b + lane; q < e; q += L) {
-      const uint2 im = __ldg(V.mem + q);
-      const uint32_t i = im.x, m = im.y;
+      const uint32_t i = __ldg(V.mem + q);
       // the cluster's record: rotation rows with the centre, then the rest
       // centre and compliance (written by k_sm_moment this iteration)
       const float4 a0 = V.rot4[4 * (size_t)i], a1 = V.rot4[4 * (size_t)i + 1], a2 = V.rot4[4 * (size_t)i + 2],
@@ -876,13 +954,13 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
       const f3 c = mk(a0.w, a1.w, a2.w);
       const f3 cb = xyz(a3);
       const float at = a3.w / dt2;
-      const f3 lo = xyz(load_unless_first(V.pair_lambda + m, it));
+      const f3 lo = xyz(load_unless_first(V.pair_lambda + q, it));
       const f3 rr = rj - cb;
       const f3 goal = mk(dot(R0, rr), dot(R1, rr), dot(R2, rr)) + c;
       const f3 C = xyz(xj) - goal;
       const float denom = wj + at;
       const f3 dl = (neg(C) - lo * at) / denom;
-      V.pair_lambda[m] = with_w(lo + dl, 0.0f);
+      if (keep) V.pair_lambda[q] = with_w(lo + dl, 0.0f);
       const f3 dx = (dl * wj) / mj;
       const float sc = sqrtf(maxc2 / fmaxf(dot(dx, dx), maxc2));
       const f3 v = dx * sc;
@@ -897,6 +975,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
     ty += __shfl_xor_sync(0xffffffffu, ty, o);
     tz += __shfl_xor_sync(0xffffffffu, tz, o);
   }
+  // the cluster centred on the particle takes its quaternion (no lane reads
+  // one in this pass; k_sm_moment's is the next to)
+  if (V.sm_qp_by_member && act && lane == L - 1 && c1 > c0) cluster_quaternion(V, j);
   if (!act || lane != 0 || !(tx | ty | tz)) return;
   bool sat = false;
   const f3 ch = ticks_change((int)tx, (int)ty, (int)tz, S->sb_inv, &sat);
@@ -904,7 +985,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
   if (sat) atomicOr(V.flags + D->scene * kNumFlags + FLAG_SOFT, 1u);
 }
 
-// shapeMatchImplicit.ts:325-401
+// Cluster quaternions whose particle is in no cluster of its own system (no
+// lane of k_sm_gather stands for it).
 __global__ void __launch_bounds__(kBlock) k_sm_qp(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
   pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -913,41 +995,7 @@ __global__ void __launch_bounds__(kBlock) k_sm_qp(WorldView V, uint32_t rank, ui
   const DevScene* S;
   if (!group_active(V, g, rank, sub, it, &D, &S)) return;
   const uint32_t i = V.grp[g];
-  if (V.csr_off[i + 1] <= V.csr_off[i]) return;
-  const float4 r0 = V.rot4[4 * (size_t)i], r1 = V.rot4[4 * (size_t)i + 1], r2 = V.rot4[4 * (size_t)i + 2];
-  const float m00 = r0.x, m01 = r0.y, m02 = r0.z, m10 = r1.x, m11 = r1.y, m12 = r1.z, m20 = r2.x, m21 = r2.y,
-              m22 = r2.z;
-  const float tr = m00 + m11 + m22;
-  float qx, qy, qz, qw;
-  if (tr > 0.0f) {
-    const float sq = 0.5f / sqrtf(tr + 1.0f);
-    qw = 0.25f / sq;
-    qx = (m21 - m12) * sq;
-    qy = (m02 - m20) * sq;
-    qz = (m10 - m01) * sq;
-  } else if (m00 > m11 && m00 > m22) {
-    const float sq = 2.0f * sqrtf(1.0f + m00 - m11 - m22);
-    qw = (m21 - m12) / sq;
-    qx = 0.25f * sq;
-    qy = (m01 + m10) / sq;
-    qz = (m02 + m20) / sq;
-  } else if (m11 > m22) {
-    const float sq = 2.0f * sqrtf(1.0f + m11 - m00 - m22);
-    qw = (m02 - m20) / sq;
-    qx = (m01 + m10) / sq;
-    qy = 0.25f * sq;
-    qz = (m12 + m21) / sq;
-  } else {
-    const float sq = 2.0f * sqrtf(1.0f + m22 - m00 - m11);
-    qw = (m10 - m01) / sq;
-    qx = (m02 + m20) / sq;
-    qy = (m12 + m21) / sq;
-    qz = 0.25f * sq;
-  }
-  const float4 q0 = V.q[i];
-  const float d = q0.x * qx + q0.y * qy + q0.z * qz + q0.w * qw;
-  const float fl = d < 0.0f ? -1.0f : 1.0f;
-  V.qp[i] = make_float4(qx * fl, qy * fl, qz * fl, qw * fl);
+  if (V.csr_off[i + 1] > V.csr_off[i]) cluster_quaternion(V, i);
 }
 
 // shapeMatch.ts:53-229: one 256-thread block per body reduces the centre of
@@ -1819,9 +1867,38 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       }
     }
   }
-  // the clusters that hold each particle: (centre id, CSR position) by member
+  // the clusters that hold each particle (their centre ids) by member
   std::vector<uint32_t> mem_off(n_ + 1, 0), mem_soft(n_, 0), mem_ids;
-  std::vector<uint2> mem;
+  std::vector<uint32_t> mem;
+  // the moment pass's clusters, and their members' ids: by warp of clusters,
+  // entry m of its 32 clusters side by side where that pads them to at most
+  // about twice their members, else cluster after cluster
+  std::vector<uint4> sm_grp(grp.size());
+  std::vector<uint32_t> sm_ids;
+  for (size_t w = 0; w < grp.size(); w += 32) {
+    const size_t e = std::min(grp.size(), w + 32);
+    uint64_t most = 0, all = 0;
+    for (size_t g = w; g < e; ++g) {
+      const uint32_t deg = csr_off[grp[g] + 1] - csr_off[grp[g]];
+      most = std::max<uint64_t>(most, deg);
+      all += deg;
+    }
+    const bool side = 32 * most <= 2 * all + 256;
+    const size_t base = sm_ids.size();
+    if (base + std::max(32 * most, all) > 0xffffffffull)
+      return fail(PF_ERR_INVALID, "SoftbodySystem: too many cluster members");
+    sm_ids.resize(base + (side ? 32 * most : all), grp[w]);
+    size_t at = base;
+    for (size_t g = w; g < e; ++g) {
+      const uint32_t from = csr_off[grp[g]], deg = csr_off[grp[g] + 1] - from;
+      const size_t first = side ? base + (g - w) : at;
+      const uint32_t stride = side ? 32u : 1u;
+      for (uint32_t m = 0; m < deg; ++m) sm_ids[first + (size_t)m * stride] = csr_idx[from + m];
+      sm_grp[g] = make_uint4(grp[g], (uint32_t)first, deg, stride);
+      at += deg;
+    }
+  }
+  bool qp_by_member = true;
   {
     for (uint32_t g = 0; g < grp.size(); ++g)
       for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) {
@@ -1855,10 +1932,13 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       const uint32_t l = (uint32_t)std::atoi(e);
       if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) mem_lanes_ = l;
     }
-    mem.assign(std::max<uint32_t>(1, mem_off[n_]), make_uint2(0, 0));
+    for (uint32_t g = 0; g < grp.size(); ++g)
+      if (csr_off[grp[g] + 1] > csr_off[grp[g]])
+        qp_by_member = qp_by_member && mem_off[grp[g] + 1] > mem_off[grp[g]] && mem_soft[grp[g]] == grp_soft[g];
+    mem.assign(std::max<uint32_t>(1, mem_off[n_]), 0u);
     std::vector<uint32_t> at(mem_off.begin(), mem_off.end() - 1);
     for (uint32_t g = 0; g < grp.size(); ++g)
-      for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) mem[at[csr_idx[m]]++] = make_uint2(grp[g], m);
+      for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) mem[at[csr_idx[m]]++] = grp[g];
   }
   // ---- chunk table and per-slot state ----------------------------------
   std::vector<uint32_t> chunk(n_ / kSegAlign, 0);
@@ -2002,7 +2082,10 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     base_.omega = need_soft ? cv.take<float4>(N) : nullptr;
     base_.pair_lambda = cv.take<float4>(csr_idx.size());
     base_.mem_off = any_soft_local_ ? cv.take<uint32_t>(N + 1) : nullptr;
-    base_.mem = any_soft_local_ ? cv.take<uint2>(mem.size()) : nullptr;
+    base_.mem = any_soft_local_ ? cv.take<uint32_t>(mem.size()) : nullptr;
+    base_.sm_grp = cv.take<uint4>(sm_grp.size());
+    base_.sm_ids = cv.take<uint32_t>(sm_ids.size());
+    base_.sm_slots = any_grid_ ? cv.take<uint32_t>(sm_ids.size()) : const_cast<uint32_t*>(base_.sm_ids);
     base_.mem_soft = any_soft_local_ ? cv.take<uint32_t>(N) : nullptr;
     base_.mem_ids = any_soft_local_ ? cv.take<uint32_t>(mem_ids.size()) : nullptr;
     base_.n_mem_ids = any_soft_local_ ? (uint32_t)mem_ids.size() : 0u;
@@ -2079,6 +2162,8 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   base_.n = n_;
   base_.prim_stride = prim_stride_;
   base_.n_grp = (uint32_t)grp.size();
+  base_.n_sm = (uint32_t)sm_ids.size();
+  base_.sm_qp_by_member = qp_by_member ? 1u : 0u;
   base_.n_bodies = (uint32_t)h_bodies_.size();
   base_.n_cons = (uint32_t)ci.size();
   base_.n_bend = (uint32_t)bidx.size();
@@ -2184,7 +2269,9 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     PF_TRY(up(base_.csr_idx, csr_idx.data(), 4 * csr_idx.size()));
     if (any_soft_local_) {
       PF_TRY(up(const_cast<uint32_t*>(base_.mem_off), mem_off.data(), 4 * mem_off.size()));
-      PF_TRY(up(const_cast<uint2*>(base_.mem), mem.data(), sizeof(uint2) * mem.size()));
+      PF_TRY(up(base_.mem, mem.data(), 4 * mem.size()));
+      PF_TRY(up(base_.sm_grp, sm_grp.data(), sizeof(uint4) * sm_grp.size()));
+      PF_TRY(up(base_.sm_ids, sm_ids.data(), 4 * sm_ids.size()));
       PF_TRY(up(const_cast<uint32_t*>(base_.mem_soft), mem_soft.data(), 4 * mem_soft.size()));
       PF_TRY(up(const_cast<uint32_t*>(base_.mem_ids), mem_ids.data(), 4 * mem_ids.size()));
     }
@@ -2897,6 +2984,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   } else {
     launch_slots(k_reset_sums, n_, stream_, V);
   }
+  if (any_soft_local_ && any_grid_) launch_slots(k_sm_slots, base_.n_sm, stream_, V);
   // the other fluid scenes' passes run over their chunks (all fluid chunks
   // without groups); the grouped scenes run after the cloth fork below
   const WorldView VF = rest_view(V);
@@ -2960,7 +3048,8 @@ void World::run_substep(uint32_t s, uint32_t parity) {
         if (rest) launch_slots(k_fluid_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s, it, slot ? 1u : 0u);
       }
       if (has_local) {
-        launch_slots(k_sm_moment, base_.n_grp, stream_, V, r, s, it);
+        launch_kernel(k_sm_moment, div_up(base_.n_grp, kSmBlock), kSmBlock, 0, stream_, V, r, s, it);
+        ++t_launches;
         if (base_.n_mem_ids) {  // mem_lanes_ lanes per cluster member
           const uint32_t grid = (uint32_t)(((uint64_t)mem_lanes_ * base_.n_mem_ids + kBlock - 1) / kBlock);
           if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kBlock, 0, stream_, V, r, s, it);
@@ -2971,7 +3060,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
           else launch_kernel(k_sm_gather<32>, grid, kBlock, 0, stream_, V, r, s, it);
           ++t_launches;
         }
-        launch_slots(k_sm_qp, base_.n_grp, stream_, V, r, s, it);
+        if (!base_.sm_qp_by_member) launch_slots(k_sm_qp, base_.n_grp, stream_, V, r, s, it);
       }
       if (has_global && base_.n_bodies) {
         launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, it, 1u);

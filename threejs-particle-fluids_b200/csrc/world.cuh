@@ -359,14 +359,21 @@ struct WorldView {
   float4* q;                 // orientation
   float4* qp;                // predicted orientation
   float4* omega;             // angular velocity
-  float4* pair_lambda;       // per CSR entry
+  float4* pair_lambda;       // per entry of mem
   // the clusters that hold each particle (by id): entries [mem_off[j],
-  // mem_off[j + 1]) of mem are (cluster centre id, CSR position), mem_soft[j]
-  // the particle's soft system
+  // mem_off[j + 1]) of mem are their centre ids, mem_soft[j] the particle's
+  // soft system
   const uint32_t* mem_off;
-  const uint2* mem;
+  const uint32_t* mem;
   const uint32_t* mem_soft;
   const uint32_t* mem_ids;   // the ids held by at least one cluster, ascending
+  // the moment pass: per cluster (id, first entry, members, entry stride) into
+  // the members' ids and their slots of this substep
+  const uint4* sm_grp;
+  const uint32_t* sm_ids;
+  uint32_t* sm_slots;
+  uint32_t n_sm;
+  uint32_t sm_qp_by_member;  // every cluster's particle is a member: k_sm_gather takes the quaternions
   uint32_t n_mem_ids;
   float4* lambda_g;          // global matching multipliers per id
   float4* body_c;            // per body
