@@ -194,3 +194,52 @@ def test_sort_in_one_cluster(oracle, n, dims):
     assert np.array_equal(a.counts, b["count"])
     assert np.array_equal(a.cell_start, b["start"])
     assert np.array_equal(a.sorted_indices, b["perm"])
+
+
+@pytest.mark.parametrize("edges", ["lattice", "star", "complete", "pair"])
+@pytest.mark.parametrize("fluid", [False, True])
+def test_cluster_layouts(oracle, edges, fluid):
+    """Shape matching over clusters of equal size, one large cluster among
+    small ones (a warp's lists laid out cluster after cluster), every particle
+    in every cluster, and particles without neighbours; in a world without a
+    grid and in one whose slots move (a fluid beside the body): the oracle's
+    positions and orientations."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    g = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3) * 0.02 + [0.3, 0.02, 0.3]
+    n = 70 if edges == "complete" else 125
+    g = g[:n]
+    if edges == "lattice":
+        d = np.abs(g[:, None] - g[None]).max(-1)
+        e = np.argwhere((d < 0.025) & (np.arange(n)[:, None] < np.arange(n)[None]))
+    elif edges == "star":
+        e = np.array([(0, k) for k in range(1, n)])
+    elif edges == "complete":
+        e = np.array([(i, j) for i in range(n) for j in range(i + 1, n)])
+    else:
+        e = np.array([(0, 1)])
+    r = np.random.default_rng(3)
+    pos = g.astype(np.float32)
+    vel = r.normal(0, 0.2, (n, 3)).astype(np.float32)
+    w = np.full(n, 1.0 / 0.008, np.float32)
+    ups, mats = [R.Upload(0, pos, vel, w)], [("soft", R.SoftbodyOpts([R.BodyDef(
+        range=(0, n), compliance=1e-5, edges=e.astype(np.uint32))], "local"))]
+    cap = n
+    if fluid:
+        f = (r.uniform(0, 0.1, (300, 3)) + [0.6, 0.05, 0.3]).astype(np.float32)
+        ups.append(R.Upload(n, f))
+        mats.append(("fluid", R.FluidOpts(range=(n, 300), particle_spacing=0.02, rest_density=1000.0, viscosity=0.01)))
+        cap += 300
+    rec = R.Recipe(capacity=cap, radius=0.01, uploads=ups, materials=mats,
+                   prims=R.container_walls((0.0, 0.0, 0.0), (1.0, 1.0, 1.0)), loop=R.LoopOpts(substeps=2, iterations=3))
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    a.step(1 / 60)
+    b.step(1 / 60)
+    # positions within 1e-5 of the container's metre; quaternions of unit
+    # length, from rotations of clusters a few centimetres wide: 1e-5 / 0.02
+    x, y = a.readback(N.PF_FIELD_POSITIONS)[:n], b.readback(N.PF_FIELD_POSITIONS)[:n]
+    assert np.abs(x - y).max() <= 1e-5
+    q, p = a.readback(N.PF_FIELD_ROTATION)[:n], b.readback(N.PF_FIELD_ROTATION)[:n]
+    assert np.abs(q - p).max() <= 5e-4
+    a.close()

@@ -777,7 +777,8 @@ __global__ void __launch_bounds__(kBlock) k_sm_slots(WorldView V) {
 // from lists laid out warp by warp (entry m of a warp's clusters is one line;
 // the slots are looked up once per substep), so that a member costs one
 // dependent load after a coalesced one, and eight (four in the moment)
-// members are in flight at a time, summed in CSR order. MOMENTTIMES
+// members are in flight at a time, summed in CSR order: 50,000 clusters of 27
+// took 18.4 us with index, slot and position chased per member, 14.7 so.
 __global__ void __launch_bounds__(kSmBlock) k_sm_moment(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
   pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -848,16 +849,17 @@ __global__ void __launch_bounds__(kSmBlock) k_sm_moment(WorldView V, uint32_t ra
   if (deg == 0) {
     r[0] = 1; r[1] = 0; r[2] = 0; r[3] = 0; r[4] = 1; r[5] = 0; r[6] = 0; r[7] = 0; r[8] = 1;
   }
-  V.rot4[4 * (size_t)i + 0] = make_float4(r[0], r[1], r[2], c.x);
-  V.rot4[4 * (size_t)i + 1] = make_float4(r[3], r[4], r[5], c.y);
-  V.rot4[4 * (size_t)i + 2] = make_float4(r[6], r[7], r[8], c.z);
-  V.rot4[4 * (size_t)i + 3] = make_float4(cb.x, cb.y, cb.z, rest_i.w);
+  const size_t n = V.n;
+  V.rot4[i] = make_float4(r[0], r[1], r[2], c.x);
+  V.rot4[n + i] = make_float4(r[3], r[4], r[5], c.y);
+  V.rot4[2 * n + i] = make_float4(r[6], r[7], r[8], c.z);
+  V.rot4[3 * n + i] = make_float4(cb.x, cb.y, cb.z, rest_i.w);
 }
 
 // shapeMatchImplicit.ts:325-401: the quaternion of cluster i's rotation, on the
 // side of its committed one.
 __device__ __forceinline__ void cluster_quaternion(const WorldView& V, uint32_t i) {
-  const float4 r0 = V.rot4[4 * (size_t)i], r1 = V.rot4[4 * (size_t)i + 1], r2 = V.rot4[4 * (size_t)i + 2];
+  const float4 r0 = V.rot4[i], r1 = V.rot4[(size_t)V.n + i], r2 = V.rot4[2 * (size_t)V.n + i];
   const float m00 = r0.x, m01 = r0.y, m02 = r0.z, m10 = r1.x, m11 = r1.y, m12 = r1.z, m20 = r2.x, m21 = r2.y,
               m22 = r2.z;
   const float tr = m00 + m11 + m22;
@@ -907,8 +909,16 @@ __device__ __forceinline__ void cluster_quaternion(const WorldView& V, uint32_t 
 // reads that position in this pass: the clusters' centres and rotations come
 // from the passes before. Every lane of a warp reaches the shuffles: a lane
 // past the last member, or whose member's body skips this pass, adds zero.
+//
+// Consecutive particles are mostly neighbours in their body, so their k-th
+// clusters are mostly consecutive: the clusters' records come as four planes
+// by cluster id, a few lines a load, where records of 64 bytes made each of
+// the four loads touch a line per particle and L1 bound the pass. A member's
+// multipliers lie side by side. 50,000 particles in 27 clusters each, step
+// with its read: 1,466 us with records, 1,374 with planes; entries and
+// multipliers laid out warp by warp as well: 1,409.
 template <uint32_t L>
-__global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
+__global__ void __launch_bounds__(kSmBlock, 8) k_sm_gather(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
   pdl_begin();
   static_assert(L == 1 || L == 2 || L == 4 || L == 8 || L == 16 || L == 32,
                 "lanes per member: a power of two dividing the warp");
@@ -919,19 +929,17 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
   const DevScene* S = nullptr;
   uint32_t tx = 0, ty = 0, tz = 0, sj = 0;
   float4 xj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  uint32_t j = 0, b = 0, e = 0, c0 = 0, c1 = 0;
+  uint32_t j = 0;
+  uint4 M = make_uint4(0, 0, 0, 0);
   float4 rest4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (act) {
     // the member's own records are loaded beside its body and scene (they
     // do not depend on them), so the chains of dependent loads overlap
-    j = __ldg(V.mem_ids + t / L);
+    M = __ldg(V.mem_info + t / L);  // id, first entry, entries, members of its own cluster
+    j = M.x;
     const uint32_t soft = V.mem_soft[j];
-    b = V.mem_off[j];
-    e = V.mem_off[j + 1];
     sj = V.inv[j];
     rest4 = V.rest[j];
-    c0 = V.csr_off[j];
-    c1 = V.csr_off[j + 1];
     D = &V.softs[soft];
     xj = V.cur.xs[sj];
     S = &V.scenes[D->scene];
@@ -940,16 +948,19 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
   if (act) {
     const f3 rj = xyz(rest4);
     const float wj = xj.w;
-    const float mj = fmaxf((float)(c1 - c0), 1.0f);
+    const float mj = fmaxf((float)M.w, 1.0f);
     const float dt2 = S->dt * S->dt;
     const float maxc2 = D->maxc2, scale = S->sb_scale;
     const bool keep = it + 1 < S->iterations;  // the multipliers are read once more
-    for (uint32_t q = b + lane; q < e; q += L) {
-      const uint32_t i = __ldg(V.mem + q);
+    const size_t n = V.n;
+    const uint32_t e = M.y + M.z;
+    uint32_t next = lane < M.z ? __ldg(V.mem + M.y + lane) : 0u;
+    for (uint32_t q = M.y + lane; q < e; q += L) {
+      const uint32_t i = next;
+      if (q + L < e) next = __ldg(V.mem + q + L);
       // the cluster's record: rotation rows with the centre, then the rest
       // centre and compliance (written by k_sm_moment this iteration)
-      const float4 a0 = V.rot4[4 * (size_t)i], a1 = V.rot4[4 * (size_t)i + 1], a2 = V.rot4[4 * (size_t)i + 2],
-                   a3 = V.rot4[4 * (size_t)i + 3];
+      const float4 a0 = V.rot4[i], a1 = V.rot4[n + i], a2 = V.rot4[2 * n + i], a3 = V.rot4[3 * n + i];
       const f3 R0 = xyz(a0), R1 = xyz(a1), R2 = xyz(a2);
       const f3 c = mk(a0.w, a1.w, a2.w);
       const f3 cb = xyz(a3);
@@ -977,7 +988,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_sm_gather(WorldView V, uint32_t r
   }
   // the cluster centred on the particle takes its quaternion (no lane reads
   // one in this pass; k_sm_moment's is the next to)
-  if (V.sm_qp_by_member && act && lane == L - 1 && c1 > c0) cluster_quaternion(V, j);
+  if (V.sm_qp_by_member && act && lane == L - 1 && M.w > 0) cluster_quaternion(V, j);
   if (!act || lane != 0 || !(tx | ty | tz)) return;
   bool sat = false;
   const f3 ch = ticks_change((int)tx, (int)ty, (int)tz, S->sb_inv, &sat);
@@ -1870,6 +1881,7 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   // the clusters that hold each particle (their centre ids) by member
   std::vector<uint32_t> mem_off(n_ + 1, 0), mem_soft(n_, 0), mem_ids;
   std::vector<uint32_t> mem;
+  std::vector<uint4> mem_info;
   // the moment pass's clusters, and their members' ids: by warp of clusters,
   // entry m of its 32 clusters side by side where that pads them to at most
   // about twice their members, else cluster after cluster
@@ -1914,19 +1926,19 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       mem_off[i + 1] += mem_off[i];
     }
     // lanes per member in k_sm_gather: the smallest power of two that takes
-    // the clusters of nine members in ten in at most sixteen rounds. Each
-    // member starts with a chain of dependent loads (its id, body, scene,
-    // slot and position), so more members per warp keep more of those chains
-    // in flight; some rounds per member cost less than idle chains. On the
-    // serving stream's soft bodies (27 clusters per member) one served tick
-    // took 15.8, 13.2, 11.8, 10.7, 10.4 and 10.9 ms with 32, 16, 8, 4, 2 and
-    // 1 lanes.
+    // the clusters of nine members in ten in at most sixteen rounds (two for
+    // the 27 clusters of a voxel body's particle), more (eight at most) while
+    // all lanes together are fewer than 65,536, which leave SMs idle. 20,000
+    // members, 1, 2, 4 and 8 lanes each: 2,147, 2,041, 1,978 and 2,004 us a
+    // step; 50,000: 1,517, 1,409, 1,448 and 1,441; 164,000: 2,479, 2,509,
+    // 2,522 and 2,693.
     mem_lanes_ = 1;
     if (!held.empty()) {
       const size_t at = (held.size() * 9) / 10;
       std::nth_element(held.begin(), held.begin() + at, held.end());
       const uint32_t p90 = held[at];
       while (mem_lanes_ < 32 && mem_lanes_ * 16 < p90) mem_lanes_ *= 2;
+      while (mem_lanes_ < 8 && mem_lanes_ < p90 && mem_lanes_ * held.size() < 65536) mem_lanes_ *= 2;
     }
     if (const char* e = std::getenv("PFSIM_MEMBER_LANES")) {  // fixed choice for measurements and tests
       const uint32_t l = (uint32_t)std::atoi(e);
@@ -1935,7 +1947,12 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     for (uint32_t g = 0; g < grp.size(); ++g)
       if (csr_off[grp[g] + 1] > csr_off[grp[g]])
         qp_by_member = qp_by_member && mem_off[grp[g] + 1] > mem_off[grp[g]] && mem_soft[grp[g]] == grp_soft[g];
-    mem.assign(std::max<uint32_t>(1, mem_off[n_]), 0u);
+    mem_info.resize(mem_ids.size());
+    mem.assign(mem_off[n_], 0u);
+    for (size_t t = 0; t < mem_ids.size(); ++t) {
+      const uint32_t id = mem_ids[t];
+      mem_info[t] = make_uint4(id, mem_off[id], mem_off[id + 1] - mem_off[id], csr_off[id + 1] - csr_off[id]);
+    }
     std::vector<uint32_t> at(mem_off.begin(), mem_off.end() - 1);
     for (uint32_t g = 0; g < grp.size(); ++g)
       for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) mem[at[csr_idx[m]]++] = grp[g];
@@ -2072,7 +2089,6 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     base_.grp = cv.take<uint32_t>(grp.size());
     base_.grp_soft = cv.take<uint32_t>(grp_soft.size());
     base_.csr_off = need_soft ? cv.take<uint32_t>(N + 1) : nullptr;
-    base_.csr_idx = cv.take<uint32_t>(csr_idx.size());
     base_.rest = need_soft ? cv.take<float4>(N) : nullptr;
     base_.rest_c = need_soft ? cv.take<float4>(N) : nullptr;
     base_.weights = need_soft ? cv.take<float>(N) : nullptr;
@@ -2080,14 +2096,13 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     base_.q = need_soft ? cv.take<float4>(N) : nullptr;
     base_.qp = need_soft ? cv.take<float4>(N) : nullptr;
     base_.omega = need_soft ? cv.take<float4>(N) : nullptr;
-    base_.pair_lambda = cv.take<float4>(csr_idx.size());
-    base_.mem_off = any_soft_local_ ? cv.take<uint32_t>(N + 1) : nullptr;
+    base_.pair_lambda = cv.take<float4>(mem.size());
     base_.mem = any_soft_local_ ? cv.take<uint32_t>(mem.size()) : nullptr;
     base_.sm_grp = cv.take<uint4>(sm_grp.size());
     base_.sm_ids = cv.take<uint32_t>(sm_ids.size());
     base_.sm_slots = any_grid_ ? cv.take<uint32_t>(sm_ids.size()) : const_cast<uint32_t*>(base_.sm_ids);
     base_.mem_soft = any_soft_local_ ? cv.take<uint32_t>(N) : nullptr;
-    base_.mem_ids = any_soft_local_ ? cv.take<uint32_t>(mem_ids.size()) : nullptr;
+    base_.mem_info = any_soft_local_ ? cv.take<uint4>(mem_info.size()) : nullptr;
     base_.n_mem_ids = any_soft_local_ ? (uint32_t)mem_ids.size() : 0u;
     base_.lambda_g = need_soft ? cv.take<float4>(N) : nullptr;
     base_.body_c = cv.take<float4>(h_bodies_.size());
@@ -2266,14 +2281,12 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   PF_TRY(up(base_.grp_soft, grp_soft.data(), 4 * grp_soft.size()));
   if (need_soft) {
     PF_TRY(up(base_.csr_off, csr_off.data(), 4 * csr_off.size()));
-    PF_TRY(up(base_.csr_idx, csr_idx.data(), 4 * csr_idx.size()));
     if (any_soft_local_) {
-      PF_TRY(up(const_cast<uint32_t*>(base_.mem_off), mem_off.data(), 4 * mem_off.size()));
       PF_TRY(up(base_.mem, mem.data(), 4 * mem.size()));
       PF_TRY(up(base_.sm_grp, sm_grp.data(), sizeof(uint4) * sm_grp.size()));
       PF_TRY(up(base_.sm_ids, sm_ids.data(), 4 * sm_ids.size()));
       PF_TRY(up(const_cast<uint32_t*>(base_.mem_soft), mem_soft.data(), 4 * mem_soft.size()));
-      PF_TRY(up(const_cast<uint32_t*>(base_.mem_ids), mem_ids.data(), 4 * mem_ids.size()));
+      PF_TRY(up(base_.mem_info, mem_info.data(), sizeof(uint4) * mem_info.size()));
     }
     PF_TRY(up(base_.rest, rest4.data(), 16 * N));
     PF_TRY(up(base_.rest_c, restc4.data(), 16 * N));
@@ -3051,13 +3064,13 @@ void World::run_substep(uint32_t s, uint32_t parity) {
         launch_kernel(k_sm_moment, div_up(base_.n_grp, kSmBlock), kSmBlock, 0, stream_, V, r, s, it);
         ++t_launches;
         if (base_.n_mem_ids) {  // mem_lanes_ lanes per cluster member
-          const uint32_t grid = (uint32_t)(((uint64_t)mem_lanes_ * base_.n_mem_ids + kBlock - 1) / kBlock);
-          if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 2) launch_kernel(k_sm_gather<2>, grid, kBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 4) launch_kernel(k_sm_gather<4>, grid, kBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 8) launch_kernel(k_sm_gather<8>, grid, kBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 16) launch_kernel(k_sm_gather<16>, grid, kBlock, 0, stream_, V, r, s, it);
-          else launch_kernel(k_sm_gather<32>, grid, kBlock, 0, stream_, V, r, s, it);
+          const uint32_t grid = (uint32_t)(((uint64_t)mem_lanes_ * base_.n_mem_ids + kSmBlock - 1) / kSmBlock);
+          if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 2) launch_kernel(k_sm_gather<2>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 4) launch_kernel(k_sm_gather<4>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 8) launch_kernel(k_sm_gather<8>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          else if (mem_lanes_ == 16) launch_kernel(k_sm_gather<16>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          else launch_kernel(k_sm_gather<32>, grid, kSmBlock, 0, stream_, V, r, s, it);
           ++t_launches;
         }
         if (!base_.sm_qp_by_member) launch_slots(k_sm_qp, base_.n_grp, stream_, V, r, s, it);

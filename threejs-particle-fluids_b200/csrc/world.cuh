@@ -348,25 +348,23 @@ struct WorldView {
   const uint32_t* grp_soft;  // soft index per group
   uint32_t n_grp;
   const uint32_t* csr_off;   // by id, n + 1
-  const uint32_t* csr_idx;
   const float4* rest;        // rest offsets, w = compliance
   const float4* rest_c;      // neighbourhood rest centres
   const float* weights;
-  // 4 rows per cluster id: the rotation's rows with the cluster centre's
-  // x, y, z in w, then (rest centre, compliance); the record the
-  // shape-matching gather reads per (member, cluster) pair, 64 aligned bytes
+  // four planes of n by cluster id: the rotation's rows with the cluster
+  // centre's x, y, z in w, then (rest centre, compliance); what the
+  // shape-matching gather reads per (member, cluster) pair
   float4* rot4;
   float4* q;                 // orientation
   float4* qp;                // predicted orientation
   float4* omega;             // angular velocity
   float4* pair_lambda;       // per entry of mem
-  // the clusters that hold each particle (by id): entries [mem_off[j],
-  // mem_off[j + 1]) of mem are their centre ids, mem_soft[j] the particle's
-  // soft system
-  const uint32_t* mem_off;
+  // the clusters that hold each particle: per member (ascending ids) its id,
+  // first entry and entries of mem (the clusters' centre ids), and the members
+  // of its own cluster; mem_soft[j] is particle j's soft system
+  const uint4* mem_info;
   const uint32_t* mem;
   const uint32_t* mem_soft;
-  const uint32_t* mem_ids;   // the ids held by at least one cluster, ascending
   // the moment pass: per cluster (id, first entry, members, entry stride) into
   // the members' ids and their slots of this substep
   const uint4* sm_grp;
