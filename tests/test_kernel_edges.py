@@ -243,3 +243,31 @@ def test_cluster_layouts(oracle, edges, fluid):
     q, p = a.readback(N.PF_FIELD_ROTATION)[:n], b.readback(N.PF_FIELD_ROTATION)[:n]
     assert np.abs(q - p).max() <= 5e-4
     a.close()
+
+
+@pytest.mark.parametrize("side", [2, 3, 12, 46])
+@pytest.mark.parametrize("fluid", [False, True])
+def test_cloth_colours_in_a_chain(oracle, side, fluid):
+    """Sheets whose colours hold one constraint, less than a block and a few
+    blocks, with bending and tethers, alone and beside a fluid whose grid
+    moves the slots between substeps: the oracle's positions within 1e-5 of
+    the container."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+    from pfsim import workloads as W
+
+    rec = W.cloth_sheet(side, seed=3, bend_compliance=1e-5, tethers=True, stretch_tolerance=0.06, wind=(0.8, 0.0, 1.5))
+    n = rec.capacity
+    if fluid:
+        r = np.random.default_rng(5)
+        f = (r.uniform(0, 0.1, (300, 3)) + [0.3, 0.05, 0.3]).astype(np.float32)
+        rec.uploads.append(R.Upload(n, f))
+        rec.materials.append(("fluid", R.FluidOpts(range=(n, 300), particle_spacing=0.02, rest_density=1000.0,
+                                                   viscosity=0.01)))
+        rec.capacity = n + 300
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    a.step(1 / 60)
+    b.step(1 / 60)
+    x, y = a.readback(N.PF_FIELD_POSITIONS)[:n], b.readback(N.PF_FIELD_POSITIONS)[:n]
+    assert np.abs(x - y).max() <= 1e-5
+    a.close()

@@ -65,15 +65,22 @@ constexpr uint32_t kLookbackSpinLimit = 1u << 24;
 // LinkedLaunches scope are therefore linked (programmatic dependent launch):
 // the next kernel's blocks are placed once the blocks of the one before have
 // exited, and wait in pdl_begin(), their first statement, until its writes
-// are visible. Nothing of a kernel runs before its pdl_begin(), so the order
-// of the work is that of plain launches. No kernel signals its dependents
-// earlier: blocks placed beside a running kernel crowded on the SMs that it
-// left first, which made the soft-body passes 7 % slower (24 mixed scenes:
-// 2.67 ms a step plain, 2.87 signalled at the start, 2.64 at the exit).
+// are visible. Nothing of a kernel runs before its pdl_begin(), apart from the
+// cloth's colours, which read what no kernel just before them writes; so the
+// order of the work is that of plain launches. Only those colours signal their
+// dependents before they end: blocks placed beside a running kernel crowded on
+// the SMs that it left first, which made the soft-body passes 7 % slower (24
+// mixed scenes: 2.67 ms a step plain, 2.87 signalled at the start, 2.64 at the
+// exit), and signalled from small grids alone, nothing got faster.
 // Plain and linked: a sort of 20,011 particles 57 and 40 us, of 1,000,003
 // 103 and 72, a 256 x 256 cloth's step (190 launches) 0.86 and 0.81 ms, a
 // 30,000-particle fluid's with surface effects (307) 2.31 and 2.24.
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel's blocks be placed while this one runs: only after
+// this kernel's own pdl_begin(), so that what the next one reads before its
+// wait is safe from every kernel but this.
+__device__ __forceinline__ void pdl_signal() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The calling thread's state: linking is on inside a scope, and the last
 // operation issued there was a kernel on `last`.

@@ -497,30 +497,40 @@ __global__ void __launch_bounds__(kBlock) k_friction(WorldView V, uint32_t sub) 
 }
 
 // ---------------------------------------------------------------- cloth ----
+constexpr int kClothBlock = 128;
 // distance.ts:264-288 for one colour of constraints (no two share a particle).
-__global__ void __launch_bounds__(kBlock) k_cloth(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
-                                                  uint32_t it) {
-  pdl_begin();
+__global__ void __launch_bounds__(kClothBlock) k_cloth(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it,
+                                                  bool early) {
+  if (!early) pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= end) return;
-  const DevScene& S = V.scenes[V.c_scene[q]];
-  if (sub >= S.substeps || it >= S.iterations) return;
-  const uint32_t i = V.inv[V.c_i[q]], j = V.inv[V.c_j[q]];
+  bool act = q < end;
+  uint32_t i = 0, j = 0;
+  float at = 0.0f, rest = 0.0f;
+  if (act) {
+    const DevScene& S = V.scenes[V.c_scene[q]];
+    act = sub < S.substeps && it < S.iterations;
+    i = V.inv[V.c_i[q]];
+    j = V.inv[V.c_j[q]];
+    at = V.c_comp[q] / (S.dt * S.dt);
+    rest = V.c_rest[q];
+  }
+  if (early) pdl_begin();
+  pdl_signal();
+  if (!act) return;
   const float4 xi = V.cur.xs[i], xj = V.cur.xs[j];
+  // the multipliers start each substep at zero (so the first iteration does
+  // not read them)
+  const float lc = it ? V.c_lambda[q] : 0.0f;
   const float wi = xi.w, wj = xj.w;
   const float ws = wi + wj;
   const f3 off = xyz(xi) - xyz(xj);
   const float l = len(off);
-  // the multipliers start each substep at zero (so the first iteration does
-  // not read them)
-  const float lc = it ? V.c_lambda[q] : 0.0f;
   if (ws <= 0.0f || l < 1e-12f) {
     if (!it) V.c_lambda[q] = 0.0f;
     return;
   }
   const f3 nrm = off / l;
-  const float at = V.c_comp[q] / (S.dt * S.dt);
-  const float dl = (-(l - V.c_rest[q]) - at * lc) / (ws + at);
+  const float dl = (-(l - rest) - at * lc) / (ws + at);
   V.cur.xs[i] = with_w(xyz(xi) + nrm * (wi * dl), wi);
   V.cur.xs[j] = with_w(xyz(xj) - nrm * (wj * dl), wj);
   V.c_lambda[q] = lc + dl;
@@ -531,14 +541,27 @@ __global__ void __launch_bounds__(kBlock) k_cloth(WorldView V, uint32_t begin, u
 // theta = atan2((N1 x N2).E, (N1.N2)|E|) with E = p2 - p1,
 // N1 = (p3 - p1) x (p3 - p2), N2 = (p4 - p2) x (p4 - p1), and the XPBD
 // multiplier update (xpbd.ts:26-36).
-__global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it) {
-  pdl_begin();
+__global__ void __launch_bounds__(kClothBlock) k_bend(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it,
+                                                 bool early) {
+  if (!early) pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= end) return;
-  const DevScene& S = V.scenes[V.b_scene[q]];
-  if (sub >= S.substeps || it >= S.iterations) return;
-  const uint4 id = V.b_idx[q];
-  const uint32_t i1 = V.inv[id.x], i2 = V.inv[id.y], i3 = V.inv[id.z], i4 = V.inv[id.w];
+  bool act = q < end;
+  uint32_t i1 = 0, i2 = 0, i3 = 0, i4 = 0;
+  float at = 0.0f, rest = 0.0f;
+  if (act) {
+    const DevScene& S = V.scenes[V.b_scene[q]];
+    act = sub < S.substeps && it < S.iterations;
+    const uint4 id = V.b_idx[q];
+    i1 = V.inv[id.x];
+    i2 = V.inv[id.y];
+    i3 = V.inv[id.z];
+    i4 = V.inv[id.w];
+    at = V.cloth_par[V.b_cloth[q]].bend_compliance / (S.dt * S.dt);
+    rest = V.b_rest[q];
+  }
+  if (early) pdl_begin();
+  pdl_signal();
+  if (!act) return;
   const float4 p1 = V.cur.xs[i1], p2 = V.cur.xs[i2], p3 = V.cur.xs[i3], p4 = V.cur.xs[i4];
   const f3 x1 = xyz(p1), x2 = xyz(p2), x3 = xyz(p3), x4 = xyz(p4);
   const f3 E = x2 - x1;
@@ -555,7 +578,7 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
   if (n1s < 1e-24f || n2s < 1e-24f) return;
   const float st = dot(cross(n1, n2), E);
   const float ct = dot(n1, n2) * el;
-  const float C = atan2f(st, ct) - V.b_rest[q];
+  const float C = atan2f(st, ct) - rest;
   const f3 N1 = n1 / n1s, N2 = n2 / n2s;
   const f3 g3 = neg(N1 * el), g4 = neg(N2 * el);
   const float c31 = dot(b3, E) / el, c32 = dot(a4, E) / el;
@@ -565,7 +588,6 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
   const float w1 = p1.w, w2 = p2.w, w3 = p3.w, w4 = p4.w;
   const float sg = dot(g1, g1) * w1 + dot(g2, g2) * w2 + dot(g3, g3) * w3 + dot(g4, g4) * w4;
   if (sg <= 1e-30f) return;
-  const float at = V.cloth_par[V.b_cloth[q]].bend_compliance / (S.dt * S.dt);
   const float dl = (-C - at * lc) / (sg + at);
   V.cur.xs[i1] = with_w(x1 + g1 * (w1 * dl), w1);
   V.cur.xs[i2] = with_w(x2 + g2 * (w2 * dl), w2);
@@ -578,29 +600,37 @@ __global__ void __launch_bounds__(kBlock) k_bend(WorldView V, uint32_t begin, ui
 // free particle). Unilateral: slack inside the rest radius (lambda reset),
 // otherwise the XPBD projection of the free particle onto the sphere about
 // its pinned anchor, read at its predicted position.
-__global__ void __launch_bounds__(kBlock) k_tether(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
-                                                   uint32_t it) {
-  pdl_begin();
+__global__ void __launch_bounds__(kClothBlock) k_tether(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
+                                                   uint32_t it, bool early) {
+  if (!early) pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= end) return;
-  const DevScene& S = V.scenes[V.t_scene[q]];
-  if (sub >= S.substeps || it >= S.iterations) return;
-  const uint4 r = V.t_rec[q];
-  const uint32_t i = V.inv[r.x];
-  const float4 xi = V.cur.xs[i];
+  bool act = q < end;
+  uint32_t i = 0, j = 0;
+  float at = 0.0f, rest = 0.0f;
+  if (act) {
+    const DevScene& S = V.scenes[V.t_scene[q]];
+    act = sub < S.substeps && it < S.iterations;
+    const uint4 r = V.t_rec[q];
+    i = V.inv[r.x];
+    j = V.inv[r.y];
+    rest = __uint_as_float(r.z);
+    at = __uint_as_float(r.w) / (S.dt * S.dt);
+  }
+  if (early) pdl_begin();
+  pdl_signal();
+  if (!act) return;
+  const float4 xi = V.cur.xs[i], xj = V.cur.xs[j];
   const float w = xi.w;
   const float lc = it ? V.t_lambda[q] : 0.0f;
   if (!it) V.t_lambda[q] = 0.0f;  // for the returns below
   if (w <= 0.0f) return;
-  const f3 d = xyz(xi) - xyz(V.cur.xs[V.inv[r.y]]);
+  const f3 d = xyz(xi) - xyz(xj);
   const float l = len(d);
-  const float rest = __uint_as_float(r.z);
   if (l <= rest) {
     V.t_lambda[q] = 0.0f;
     return;
   }
   if (l < 1e-12f) return;
-  const float at = __uint_as_float(r.w) / (S.dt * S.dt);
   const float dl = (-(l - rest) - at * lc) / (w + at);
   V.cur.xs[i] = with_w(xyz(xi) + (d / l) * (w * dl), w);
   V.t_lambda[q] = lc + dl;
@@ -2958,25 +2988,23 @@ void World::run_init_pass() {
   launch_slots(k_boundary_volume, n_, stream_, view(parity_), 1u, 0u);
 }
 
-// ClothSystem.ts:193-212: the stretch colours, then the bending colours.
+// ClothSystem.ts:193-212: the stretch colours, the bending colours, the
+// tethers. All but the first follow a kernel that writes only positions and
+// multipliers, so slots and scenes can be read before it has ended.
 void World::launch_cloth_rank(const WorldView& V, uint32_t r, uint32_t s, uint32_t it, cudaStream_t st) {
-  for (auto& rg : cloth_ranges_[r])
-    if (rg.second > rg.first) {
-      launch_kernel(k_cloth, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
-      ++t_launches;
-    }
+  bool early = false;
+  const auto colour = [&](auto kernel, const std::pair<uint32_t, uint32_t>& rg) {
+    if (rg.second <= rg.first) return;
+    const uint32_t grid = div_up(rg.second - rg.first, kClothBlock);
+    launch_kernel(kernel, grid, kClothBlock, 0, st, V, rg.first, rg.second, s, it, early);
+    ++t_launches;
+    early = true;
+  };
+  for (auto& rg : cloth_ranges_[r]) colour(k_cloth, rg);
   if (r < bend_ranges_.size())
-    for (auto& rg : bend_ranges_[r])
-      if (rg.second > rg.first) {
-        launch_kernel(k_bend, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
-        ++t_launches;
-      }
+    for (auto& rg : bend_ranges_[r]) colour(k_bend, rg);
   if (r < teth_ranges_.size())
-    for (auto& rg : teth_ranges_[r])
-      if (rg.second > rg.first) {
-        launch_kernel(k_tether, div_up(rg.second - rg.first, kBlock), kBlock, 0, st, V, rg.first, rg.second, s, it);
-        ++t_launches;
-      }
+    for (auto& rg : teth_ranges_[r]) colour(k_tether, rg);
 }
 
 void World::launch_aero(const WorldView& V, uint32_t stage, uint32_t s) {
