@@ -271,3 +271,29 @@ def test_cloth_colours_in_a_chain(oracle, side, fluid):
     x, y = a.readback(N.PF_FIELD_POSITIONS)[:n], b.readback(N.PF_FIELD_POSITIONS)[:n]
     assert np.abs(x - y).max() <= 1e-5
     a.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 257, 3000])
+@pytest.mark.parametrize("quiet", [False, True])
+def test_contact_lanes(oracle, n, quiet):
+    """Crowded particles, so that rows hold more candidates and slots more
+    pairs than a slot has lanes, with collision groups, pinned particles and,
+    in half the worlds, a range that emits no pairs: the oracle's pairs, and
+    its positions within 1e-5 of the box after the pairs' solve."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    r, rng = 0.02, np.random.default_rng(7 * n + quiet)
+    side = (n * 4.19 * (2.2 * r) ** 3 / 16) ** (1 / 3)  # sixteen particles in reach of one
+    pos = rng.uniform(0, side, (n, 3)).astype(np.float32)
+    rec = K.particles(pos, r, 1, 2, gravity=(0, 0, 0), inv_mass=(rng.random(n) > 0.2).astype(np.float32),
+                      group=rng.integers(0, 4, n), contact=(64 * n, 0.5, 0.4),
+                      quiet=[(n // 4, n // 4)] if quiet and n >= 4 else [])
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend(precision=32).build(rec)
+    a.step(K.DT)
+    b.step(K.DT)
+    (ca, pa), (cb, pb) = a.contacts(), b.contacts()
+    assert ca == cb and {tuple(p) for p in pa.tolist()} == {tuple(p) for p in pb.tolist()}
+    x, y = a.readback(N.PF_FIELD_POSITIONS)[:, :3], b.readback(N.PF_FIELD_POSITIONS)[:, :3]
+    assert np.abs(x - y).max() <= 1e-5 * max(1.0, side)
+    a.close()

@@ -1236,6 +1236,15 @@ void launch_slots(K kernel, uint32_t n, cudaStream_t st, A... args) {
   ++t_launches;
 }
 
+// A contact pair pass: kPairLanes threads per slot (whole blocks, since the
+// slots come in chunks of kSegAlign).
+template <typename K, typename... A>
+void launch_pairs(K kernel, cudaStream_t st, const WorldView& V, A... args) {
+  static_assert(kSegAlign * kPairLanes % kBlock == 0, "whole blocks");
+  launch_kernel(kernel, V.n / (kBlock / kPairLanes), kBlock, 0, st, V, args...);
+  ++t_launches;
+}
+
 size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 
 // The slot neighbour passes use no shared memory and gather their
@@ -2161,15 +2170,14 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     cloth_par_dev_ = cv.take<DevCloth>(h_cloth_par_.size());
     base_.cloth_par = cloth_par_dev_;
     // particle contacts
-    const size_t CH = N / kSegAlign;
     base_.cgroup = any_contact_ ? cv.take<uint32_t>(N) : nullptr;
     base_.cquiet = any_contact_ ? cv.take<uint8_t>(N) : nullptr;
     base_.con_nbr = any_contact_ ? cv.take<uint32_t>(kMaxContacts * N) : nullptr;
     base_.con_cnt = any_contact_ ? cv.take<uint32_t>(N) : nullptr;
     base_.con_pre = any_contact_ ? cv.take<uint32_t>(N) : nullptr;
-    base_.chunk_sum = any_contact_ ? cv.take<uint32_t>(CH) : nullptr;
-    base_.chunk_drop = any_contact_ ? cv.take<uint32_t>(CH) : nullptr;
-    base_.chunk_off = any_contact_ ? cv.take<uint32_t>(CH) : nullptr;
+    base_.con_sum = any_contact_ ? cv.take<uint32_t>(N / kConGroup) : nullptr;
+    base_.con_drop = any_contact_ ? cv.take<uint32_t>(N / kConGroup) : nullptr;
+    base_.con_off = any_contact_ ? cv.take<uint32_t>(N / kConGroup) : nullptr;
     base_.con_lam = any_contact_ ? cv.take<int2>(kMaxContacts * N) : nullptr;
     base_.con_nrm = any_contact_ ? cv.take<float4>(kMaxContacts * N) : nullptr;
     base_.acc_con = any_contact_ ? cv.take<int4>(N) : nullptr;
@@ -2357,6 +2365,7 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
         cg[base + i] = sp.group[i];
         cq[base + i] = 0;
       }
+      any_quiet_ = any_quiet_ || (h_scenes_[s].contact && (!sp.fluids.empty() || !sp.quiet.empty()));
       for (auto& f : sp.fluids)
         for (uint32_t i = f.range.start; i < f.range.start + f.range.count; ++i) cq[base + i] = 1;
       for (auto& q : sp.quiet)
@@ -3032,9 +3041,9 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   // preSolve: contacts first (loop.ts:196-223), then the materials'
   if (any_contact_) {
     const uint32_t K = (uint32_t)h_scenes_.size();
-    launch_kernel(k_con_gen, n_ / kBlock, kBlock, 0, stream_, V, s);
+    launch_kernel(any_quiet_ ? k_con_gen<true> : k_con_gen<false>, n_ / kConGroup, kConBlock, 0, stream_, V, s);
     launch_kernel(k_con_scan, K, 1024, 0, stream_, V, s);
-    launch_slots(k_con_stab, n_, stream_, V, s);
+    launch_pairs(k_con_stab, stream_, V, s);
     launch_slots(k_con_apply2, n_, stream_, V, s);
     t_launches += 2;
   }
@@ -3066,7 +3075,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
     break_link();
     for (uint32_t it = 0; it < max_iter_; ++it) {
       for (uint32_t r = 0; r < cloth_ranges_.size(); ++r) launch_cloth_rank(V, r, s, it, side_stream_);
-      if (any_contact_) launch_slots(k_con_solve, n_, side_stream_, V, s, it);
+      if (any_contact_) launch_pairs(k_con_solve, side_stream_, V, s, it);
       if (any_unfused_prims_) launch_slots(k_collide, base_.n_cchunk * kSegAlign, side_stream_, V, s, it);
     }
   }
@@ -3110,7 +3119,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
       }
       if (!fork && r < cloth_ranges_.size()) launch_cloth_rank(V, r, s, it, stream_);
     }
-    if (!fork && any_contact_) launch_slots(k_con_solve, n_, stream_, V, s, it);
+    if (!fork && any_contact_) launch_pairs(k_con_solve, stream_, V, s, it);
     if (!fork && any_unfused_prims_) launch_slots(k_collide, base_.n_cchunk * kSegAlign, stream_, V, s, it);
   }
   if (fork) {
@@ -3148,7 +3157,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
   }
   // friction: the velocity sums reset, contact friction, collider friction,
   // applied (loop.ts:226-230)
-  if (any_contact_) launch_slots(k_con_friction, n_, stream_, V, s);
+  if (any_contact_) launch_pairs(k_con_friction, stream_, V, s);
   if (any_prims_ || any_contact_) launch_slots(k_friction, n_, stream_, V, s);
   if (any_prims_) {
     const uint32_t K = (uint32_t)h_scenes_.size();
@@ -3675,18 +3684,18 @@ pf_status World::contacts(uint32_t scene, uint32_t* pairs, uint32_t capacity, ui
   const uint32_t seg = S.seg_end - S.seg_start;
   uint2 st;
   PF_CUDA(cudaMemcpy(&st, base_.con_stat + scene, sizeof(uint2), cudaMemcpyDeviceToHost));
-  std::vector<uint32_t> ids(seg), cnt(seg), pre(seg), off(seg / kSegAlign), nb((size_t)kMaxContacts * seg);
+  std::vector<uint32_t> ids(seg), cnt(seg), pre(seg), off(seg / kConGroup), nb((size_t)kMaxContacts * seg);
   PF_CUDA(cudaMemcpy(ids.data(), base_.ids + S.seg_start, 4ull * seg, cudaMemcpyDeviceToHost));
   PF_CUDA(cudaMemcpy(cnt.data(), base_.con_cnt + S.seg_start, 4ull * seg, cudaMemcpyDeviceToHost));
   PF_CUDA(cudaMemcpy(pre.data(), base_.con_pre + S.seg_start, 4ull * seg, cudaMemcpyDeviceToHost));
-  PF_CUDA(cudaMemcpy(off.data(), base_.chunk_off + S.seg_start / kSegAlign, 4ull * off.size(), cudaMemcpyDeviceToHost));
+  PF_CUDA(cudaMemcpy(off.data(), base_.con_off + S.seg_start / kConGroup, 4ull * off.size(), cudaMemcpyDeviceToHost));
   for (uint32_t m = 0; m < kMaxContacts; ++m)
     PF_CUDA(cudaMemcpy(nb.data() + (size_t)m * seg, base_.con_nbr + (size_t)m * n_ + S.seg_start, 4ull * seg,
                        cudaMemcpyDeviceToHost));
   std::vector<std::pair<uint32_t, uint32_t>> out;
   for (uint32_t k = 0; k < seg; ++k) {
     const uint32_t c = std::min(cnt[k], kMaxContacts);
-    const uint32_t first = off[k / kSegAlign] + pre[k];
+    const uint32_t first = off[k / kConGroup] + pre[k];
     for (uint32_t m = 0; m < c && first + m < S.max_contacts; ++m) {
       const uint32_t a = ids[k] - S.seg_start, b = ids[nb[(size_t)m * seg + k] - S.seg_start] - S.seg_start;
       out.push_back({std::min(a, b), std::max(a, b)});

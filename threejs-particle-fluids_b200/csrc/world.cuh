@@ -59,6 +59,7 @@ __host__ __device__ __forceinline__ size_t nbr16_at(size_t k, uint32_t m) {
 __host__ __device__ __forceinline__ size_t nbr16_col(size_t k) { return nbr16_at(k, 0); }
 constexpr uint32_t kBlock = 256;
 constexpr uint64_t kSortCellCap = 0x7fffffffull;  // keys of a world's sort stay below this
+constexpr uint32_t kConGroup = 32;     // slots whose contact pairs are numbered together
 constexpr uint32_t kMaxContacts = 32;  // contact pairs kept per emitting particle per substep
 
 // ------------------------------------------------------------- host spec ----
@@ -416,10 +417,10 @@ struct WorldView {
   const uint8_t* cquiet;    // 1: inside a noSelfContacts range, by id
   uint32_t* con_nbr;
   uint32_t* con_cnt;        // pairs found per slot (uncapped)
-  uint32_t* con_pre;        // exclusive prefix of con_cnt inside the slot's 256-slot chunk
-  uint32_t* chunk_sum;      // per chunk: pairs found, and pairs past the per-slot cap
-  uint32_t* chunk_drop;
-  uint32_t* chunk_off;      // per chunk: first pair index inside its scene
+  uint32_t* con_pre;        // exclusive prefix of con_cnt inside the slot's group of kConGroup slots
+  uint32_t* con_sum;        // per group: pairs found, and pairs past the per-slot cap
+  uint32_t* con_drop;
+  uint32_t* con_off;        // per group: first pair index inside its scene
   int2* con_lam;            // (lambda_n, lambda_t) ticks of 2^-20 kg m
   float4* con_nrm;
   int4* acc_con;            // fixed-point position (then velocity) sums per slot
@@ -580,6 +581,7 @@ class World {
   bool any_react_ = false;
   bool any_unfused_prims_ = false;  // a scene whose colliders run in their own pass
   bool any_contact_ = false;        // a scene with particle contacts
+  bool any_quiet_ = false;          // one of those with a noSelfContacts range
   bool any_multi_fluid_ = false;    // a scene with two or more fluids (slot path only)
   bool fuse_dens_ = false;          // the slot list build forms the first density and lambda
   // single-fluid scenes (DevScene::grouped candidates): their chunks are
