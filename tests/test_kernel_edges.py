@@ -297,3 +297,31 @@ def test_contact_lanes(oracle, n, quiet):
     x, y = a.readback(N.PF_FIELD_POSITIONS)[:, :3], b.readback(N.PF_FIELD_POSITIONS)[:, :3]
     assert np.abs(x - y).max() <= 1e-5 * max(1.0, side)
     a.close()
+
+
+@pytest.mark.parametrize("m", [1, 15, 33, 600])
+@pytest.mark.parametrize("static", [True, False])
+def test_boundary_volume_lanes(oracle, m, static):
+    """Boundaries of one particle up to several hundred in a few cells, so
+    that a row holds less than one round of a slot's lanes, and several: the
+    oracle's volumes within 64 float roundings (a sum of some hundred
+    positive terms and one quotient)."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    rng, s, nf = np.random.default_rng(m), 0.02, 64
+    f = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3) * s + [0.3, 0.3, 0.3]
+    b = rng.uniform(0, 0.08, (m, 3)) + [0.3, 0.2, 0.3]
+    pos = np.concatenate([f, b]).astype(np.float32)
+    rec = R.Recipe(capacity=nf + m, radius=0.01,
+                   uploads=[R.Upload(0, pos, np.zeros_like(pos), np.r_[np.full(nf, 125.0), np.zeros(m)].astype(np.float32))],
+                   materials=[("fluid", R.FluidOpts(range=(0, nf), particle_spacing=s, rest_density=1000.0,
+                                                    viscosity=0.01, boundaries=[(nf, m)], boundary_static=[static]))],
+                   prims=R.container_walls((0.0, 0.0, 0.0), (1.0, 1.0, 1.0)),
+                   loop=R.LoopOpts(substeps=1, iterations=2))
+    a, o = R.NativeBackend().build(rec), oracle.OracleBackend(precision=32).build(rec)
+    a.step(1 / 60)
+    o.step(1 / 60)
+    x, y = (w.readback(N.PF_FIELD_BOUNDARY_VOLUME)[nf:].astype(np.float64) for w in (a, o))
+    assert (y > 0).all() and (np.abs(x - y) <= 64 * 2.0**-23 * y).all()
+    a.close()
