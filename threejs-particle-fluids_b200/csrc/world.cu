@@ -3284,6 +3284,16 @@ pf_status World::step(double dt) {
 // Windows past 2^27 cells stay as they are (their keys clamp and flag).
 pf_status World::maybe_grow_windows() {
   if (!any_grid_ || steps_done_ == 0) return PF_OK;
+  // A recorded step costs the host microseconds, so a caller that reads
+  // nothing between steps runs ahead of the bounds, and a window that fits
+  // the particles closely would be outgrown, and clamp, before they arrive.
+  // A plain scene therefore waits for the step before's bounds while a window
+  // is less than twice its particles' spread, and else for those of the step
+  // before that one, which leaves the GPU a step to work on meanwhile.
+  if (lazy_graph_ && steps_done_ >= kGraphAfter) {
+    const uint64_t t = steps_done_ - (windows_tight_ ? 1 : 2);
+    if (t + 1 > bounds_seen_) PF_CUDA(cudaEventSynchronize(ev_bounds_[t % kBoundsRing]));
+  }
   // the newest step whose bounds have landed (the ring holds the last
   // kBoundsRing steps; one that is still queued is skipped, not waited for)
   uint64_t seen_step = 0;
@@ -3305,7 +3315,7 @@ pf_status World::maybe_grow_windows() {
   const uint64_t since = bounds_seen_ ? seen_step + 1 - bounds_seen_ : 1;  // steps since the last look
   bounds_seen_ = seen_step + 1;
   const int32_t* seen = h_pinned_bbox_ + 6 * h_scenes_.size() * (seen_step % kBoundsRing);
-  bool any = false;
+  bool any = false, tight = false;
   for (uint32_t s = 0; s < h_scenes_.size(); ++s) {
     DevScene& S = h_scenes_[s];
     if (!S.has_grid) continue;
@@ -3321,6 +3331,7 @@ pf_status World::maybe_grow_windows() {
       // over the steps from these bounds to the end of the next one, and
       // one step more; a fluid that walls hold stops growing there
       const int64_t ext = mx - mn + 1;
+      tight = tight || 2 * ext + 8 > d;
       int32_t& prev = grow_prev_ext_[3 * s + a];
       const int64_t rate = prev > 0 ? (std::max<int64_t>(0, ext - prev) + (int64_t)since - 1) / (int64_t)since : 0;
       prev = (int32_t)ext;
@@ -3348,6 +3359,7 @@ pf_status World::maybe_grow_windows() {
     S.prune_slack = f32(big * (1.0 / 65536.0) + 1e-9);
     any = true;
   }
+  windows_tight_ = tight;
   if (!any) return PF_OK;
   return relayout_grid();
 }

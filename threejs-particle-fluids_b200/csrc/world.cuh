@@ -657,6 +657,7 @@ class World {
   cudaEvent_t ev_bounds_[kBoundsRing] = {};
   uint64_t steps_done_ = 0;
   uint64_t bounds_seen_ = 0;  // steps_done_ of the last bounds looked at, plus one (0: none yet)
+  bool windows_tight_ = true;  // a window was less than twice its particles' spread in the bounds last seen
   // Per-step parameters go through a ring of kParamRing pinned staging
   // buffers, so the host can queue that many steps ahead; a buffer is
   // written again once the event of its last upload has passed.
