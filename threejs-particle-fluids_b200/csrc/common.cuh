@@ -72,9 +72,11 @@ constexpr uint32_t kLookbackSpinLimit = 1u << 24;
 // the SMs that it left first, which made the soft-body passes 7 % slower (24
 // mixed scenes: 2.67 ms a step plain, 2.87 signalled at the start, 2.64 at the
 // exit), and signalled from small grids alone, nothing got faster.
-// Plain and linked: a sort of 20,011 particles 57 and 40 us, of 1,000,003
-// 103 and 72, a 256 x 256 cloth's step (190 launches) 0.86 and 0.81 ms, a
-// 30,000-particle fluid's with surface effects (307) 2.31 and 2.24.
+// Plain and linked, each with the kernels of its time: a sort of 20,011
+// particles 57 and 40 us (25 now, in one cluster), of 1,000,003 103 and 72, a
+// 256 x 256 cloth's step (190 launches) 0.86 and 0.81 ms (0.64 now, see
+// k_cloth), a 30,000-particle fluid's with surface effects 2.31 and 2.24
+// (1.78 now, for other reasons).
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Lets the next kernel's blocks be placed while this one runs: only after

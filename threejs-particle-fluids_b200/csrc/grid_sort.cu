@@ -3,14 +3,16 @@
 // Replaces the reference's 8-kernel HashGrid rebuild (src/core/hashGrid/
 // cellIndex.ts:113-170, sort.ts:72-192): the reference's histogram ->
 // exclusive scan -> scatter becomes, for B200,
-//   * keys with every radix pass's digit counts, from shared-memory
-//     histograms (one global atomic per digit per block);
-//   * one least-significant-digit radix pass per 11 key bits (two for a
-//     128^3 grid), each three steps: every tile of 4096 elements counts its
-//     digits; the counts are scanned over the tiles per digit (in chunks of
-//     32 tiles, then over the chunks); every tile ranks its elements by digit
-//     in element order with warp-aggregated ranks (__match_any_sync) and
-//     writes them out run by run through shared memory. The passes are
+//   * up to 65,536 elements, everything after the keys in one launch of a
+//     16-block cluster (k_small_sort);
+//   * past that, keys with every radix pass's digit counts, from
+//     shared-memory histograms (one global atomic per digit per block), and
+//     one least-significant-digit radix pass per 7 or 8 key bits, each three
+//     steps: every tile of 4096 elements counts its digits; the counts are
+//     scanned over the tiles per digit (in chunks of 32 tiles, then over the
+//     chunks); every tile ranks its elements by digit in element order with
+//     warp-aggregated ranks (a ballot per digit bit) and writes them out run
+//     by run through shared memory. The passes are
 //     stable, unlike the reference's atomic write cursor (sort.ts:187-192),
 //     so the permutation lists each cell's particles in ascending index;
 //   * cell counts from the sorted keys (one atomic per run of equal keys in a

@@ -7,7 +7,7 @@
 // partner list (column-major, entry m of slot k at m * n + k, at most
 // kMaxContacts), and a per-scene prefix over the slots numbers the pairs in
 // slot order: the first max_contacts pairs of that order are solved. Each
-// pair's multipliers and normal belong to the one thread of its emitting
+// pair's multipliers and normal belong to one lane of its emitting
 // slot, and the position and velocity corrections are fixed-point sums, so
 // the results do not depend on which side of a pair emits it (swapping the
 // pair negates every vector exactly) nor on the order of the atomic adds.
