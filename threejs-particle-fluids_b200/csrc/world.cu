@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fluid_apply(WorldView V, uint32_t
   uint32_t tg = 0;
   float4 x = make_float4(0, 0, 0, 0), d = make_float4(0, 0, 0, 0);
   if (live) {
-    tg = __ldg(V.cur.tag + k);
+    tg = V.cur.tag[k];
     x = V.cur.xs[k];
     d = V.dx[k];
   }

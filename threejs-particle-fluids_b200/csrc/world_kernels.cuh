@@ -233,8 +233,8 @@ __device__ __forceinline__ void bbox_block_add(const WorldView& V, const DevScen
 // linear keys the three cells of one (dy, dz) row are consecutive keys, so a
 // row is one contiguous slot range: row(first, end) per row.
 template <typename F>
-__device__ __forceinline__ void walk27_rows(const DevScene& S, const uint32_t* __restrict__ cstart,
-                                            const uint32_t* __restrict__ ccount, f3 p, F&& row) {
+__device__ __forceinline__ void walk27_rows(const DevScene& S, const uint32_t* cstart, const uint32_t* ccount, f3 p,
+                                            F&& row) {
   int32_t cx, cy, cz;
   local_cell(S, p, &cx, &cy, &cz, nullptr);
   const int32_t x0 = max(cx - 1, 0), x1 = min(cx + 1, (int32_t)S.dims[0] - 1);
@@ -246,8 +246,8 @@ __device__ __forceinline__ void walk27_rows(const DevScene& S, const uint32_t* _
     rs[r] = re[r] = 0;
     if (z < 0 || z >= (int32_t)S.dims[2] || y < 0 || y >= (int32_t)S.dims[1]) continue;
     const uint32_t at = S.cell_base + S.dims[0] * ((uint32_t)y + S.dims[1] * (uint32_t)z);
-    rs[r] = __ldg(cstart + at + x0);
-    re[r] = __ldg(cstart + at + x1) + __ldg(ccount + at + x1);
+    rs[r] = cstart[at + x0];
+    re[r] = cstart[at + x1] + ccount[at + x1];
   }
 #pragma unroll
   for (int r = 0; r < 9; ++r) row(rs[r], re[r]);

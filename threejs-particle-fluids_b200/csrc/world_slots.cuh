@@ -24,26 +24,30 @@
 
 namespace pf {
 
-// A list entry, or 2, 4 or 8 16-bit entries of one group (read-only for the
-// kernel; volatile, so that none moves ahead of pdl_begin()). A miss fetches
-// 256 bytes into L2: with the warp-blocked layout that is the warp's
-// neighbouring entries too.
+// What the gathers below read, another kernel of the same step has written,
+// and a linked kernel is resident before that write is visible. Their loads
+// are therefore plain ones: __ldg and ld.global.nc are for data that nobody
+// writes while the kernel lives, and are kept for the tables made at build.
+
+// A list entry, or 2, 4 or 8 16-bit entries of one group (volatile, so that
+// none moves ahead of pdl_begin()). A miss fetches 256 bytes into L2: with
+// the warp-blocked layout that is the warp's neighbouring entries too.
 __device__ __forceinline__ uint32_t ld_entry(const uint32_t* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L2::256B.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 template <uint32_t kN>
 __device__ __forceinline__ void ld_group(const uint16_t* p, uint32_t (&w)[kN / 2]) {
   static_assert(kN == 2 || kN == 4 || kN == 8, "2, 4 or 8 entries");
   if constexpr (kN == 8)
-    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
         : "l"(p));
   else if constexpr (kN == 4)
-    asm volatile("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
+    asm volatile("ld.global.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
   else
-    asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(w[0]) : "l"(p));
+    asm volatile("ld.global.L2::256B.u32 %0, [%1];" : "=r"(w[0]) : "l"(p));
 }
 
 // The list of slot k: its warp's base (kNbrWide: 32-bit entries) and the
@@ -54,8 +58,7 @@ struct NbrList {
   const uint16_t* w16;  // entry m at w16[(m / 8) * 256 + m % 8]
   __device__ __forceinline__ bool wide() const { return (base & kNbrWide) != 0; }
   __device__ __forceinline__ uint32_t entry(uint32_t m) const {
-    return wide() ? __ldg(w32 + m * kNbrStride)
-                  : base + __ldg(w16 + (m / kNbrGroup) * (kNbrStride * kNbrGroup) + m % kNbrGroup);
+    return wide() ? w32[m * kNbrStride] : base + w16[(m / kNbrGroup) * (kNbrStride * kNbrGroup) + m % kNbrGroup];
   }
 };
 __device__ __forceinline__ NbrList nbr_list(const WorldView& V, uint32_t k) {
@@ -119,7 +122,7 @@ __device__ __forceinline__ void walk_list(Entries entries, uint32_t cnt, Fetch f
 // walk_list over slot k's list in whichever width its warp stored (a
 // warp-uniform branch): 16-bit entries a group at a time. kFresh: the list
 // was written by this same thread in this kernel, so its entries are read
-// with plain (coherent) loads.
+// with loads that the compiler keeps behind those writes.
 template <uint32_t kU, bool kFresh = false, typename Fetch, typename Use>
 __device__ __forceinline__ void walk_nbrs(const NbrList& L, uint32_t cnt, Fetch fetch, Use use) {
   static_assert(kNbrGroup % kU == 0, "a round lies in one group");
@@ -260,11 +263,11 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 128 : 64) k_s_neighbors(WorldView 
   const bool dens = kDens && F.rank == 0 && S.iterations > 0;
   float rho = 0.0f, gss = 0.0f;
   f3 gs = mk(0.0f, 0.0f, 0.0f);
-  const float* __restrict__ q_of = reinterpret_cast<const float*>(V.lm) + 1;
+  const float* q_of = reinterpret_cast<const float*>(V.lm) + 1;
   const float qh = -S.homog_mass;
   const bool homog = S.homog;
   // a neighbour's record and terms for that density
-  auto fetch = [&](uint32_t j) { return NbrXQ{__ldg(V.cur.xs + j), homog ? qh : __ldg(q_of + 2 * (size_t)j)}; };
+  auto fetch = [&](uint32_t j) { return NbrXQ{V.cur.xs[j], homog ? qh : q_of[2 * (size_t)j]}; };
   auto use = [&](uint32_t, const NbrXQ& r) { lambda_terms(F, xi, r.x, r.q, rho, gs, gss); };
   const float hsq = F.hsq;
   int32_t cx, cy, cz;
@@ -303,8 +306,8 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 128 : 64) k_s_neighbors(WorldView 
       if (can_r && perp + gr * gr >= hsq) a1 = cx;
     }
     const uint32_t row = S.cell_base + S.dims[0] * ((uint32_t)y + S.dims[1] * (uint32_t)z);
-    rs[r] = __ldg(V.cstart + row + a0);
-    re[r] = __ldg(V.cstart + row + a1) + __ldg(V.ccount + row + a1);
+    rs[r] = V.cstart[row + a0];
+    re[r] = V.cstart[row + a1] + V.ccount[row + a1];
   }
   // every lane takes part in the warp's reach; then lanes of other materials
   // (f == 0) leave
@@ -335,7 +338,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 128 : 64) k_s_neighbors(WorldView 
     for (; j + kNbrUnroll <= e; j += kNbrUnroll) {
       float4 xj[kNbrUnroll];
 #pragma unroll
-      for (uint32_t q = 0; q < kNbrUnroll; ++q) xj[q] = __ldg(V.cur.xs + j + q);
+      for (uint32_t q = 0; q < kNbrUnroll; ++q) xj[q] = V.cur.xs[j + q];
 #pragma unroll
       for (uint32_t q = 0; q < kNbrUnroll; ++q) test(j + q, dist2_rn(xi, xj[q]) < hsq);
     }
@@ -343,7 +346,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 128 : 64) k_s_neighbors(WorldView 
       float4 xj[kNbrUnroll];
 #pragma unroll
       for (uint32_t q = 0; q < kNbrUnroll; ++q)
-        if (j + q < e) xj[q] = __ldg(V.cur.xs + j + q);
+        if (j + q < e) xj[q] = V.cur.xs[j + q];
 #pragma unroll
       for (uint32_t q = 0; q < kNbrUnroll; ++q)
         if (j + q < e) test(j + q, dist2_rn(xi, xj[q]) < hsq);
@@ -451,16 +454,16 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 80 : 48) k_s_lambda(WorldView V, u
   const uint32_t cnt = V.ncount[k];
   const NbrList nl = nbr_list(V, k);
   prefetch_list(nl, cnt);
-  const float* __restrict__ q_of = reinterpret_cast<const float*>(V.lm) + 1;  // lm[j].y
+  const float* q_of = reinterpret_cast<const float*>(V.lm) + 1;  // lm[j].y
   if (S.homog) {
     // one fluid, one mass: no mass gather
     const float qh = -S.homog_mass;
     walk_nbrs<kNbrUnroll>(
-        nl, cnt, [&](uint32_t j) { return __ldg(V.cur.xs + j); },
+        nl, cnt, [&](uint32_t j) { return V.cur.xs[j]; },
         [&](uint32_t, const float4& xj) { lambda_terms(F, xi, xj, qh, rho, gs, gss); });
   } else {
     walk_nbrs<kNbrUnroll>(
-        nl, cnt, [&](uint32_t j) { return NbrXQ{__ldg(V.cur.xs + j), __ldg(q_of + 2 * (size_t)j)}; },
+        nl, cnt, [&](uint32_t j) { return NbrXQ{V.cur.xs[j], q_of[2 * (size_t)j]}; },
         [&](uint32_t, const NbrXQ& r) { lambda_terms(F, xi, r.x, r.q, rho, gs, gss); });
   }
   finish_lambda(V, S, F, k, xi4, rho, gs, gss);
@@ -499,7 +502,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, ui
   prefetch_list(nl, cnt);
   auto one = [&](uint32_t j, float4 xj, float2 lq) {
     const float bvj = lq.y;
-    const float lj = (multi && tag_fluid(__ldg(V.cur.tag + j)) != f) ? 0.0f : lq.x;
+    const float lj = (multi && tag_fluid(V.cur.tag[j]) != f) ? 0.0f : lq.x;
     const float mass = code_mass(bvj, F.rho0);
     const f3 off = xi - xyz(xj);
 #ifdef PF_EXACT_ROUNDING
@@ -517,7 +520,7 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, ui
       // Is j on one of this fluid's boundaries? Its tag names the last added
       // boundary that holds it (zero: none does), which decides unless that
       // one is another fluid's; only then the fluid's ranges are searched.
-      const uint32_t tb = tag_bnd(__ldg(V.cur.tag + j));
+      const uint32_t tb = tag_bnd(V.cur.tag[j]);
       bool in = tb != 0 && tb - 1u - F.bnd_first < F.bnd_count;
       if (tb != 0 && !in) {
         const uint32_t idj = V.ids[j];
@@ -533,11 +536,11 @@ __global__ void __maxnreg__(kNbrUnroll == 8 ? 96 : 56) k_s_delta(WorldView V, ui
     // one fluid, one mass: (x*, lambda) of a neighbour in one gather
     const float qh = -S.homog_mass;
     walk_nbrs<kNbrUnroll>(
-        nl, cnt, [&](uint32_t j) { return __ldg(V.xl + j); },
+        nl, cnt, [&](uint32_t j) { return V.xl[j]; },
         [&](uint32_t j, const float4& xj) { one(j, xj, make_float2(xj.w, qh)); });
   } else {
     walk_nbrs<kNbrUnroll>(
-        nl, cnt, [&](uint32_t j) { return NbrXL{__ldg(V.cur.xs + j), __ldg(V.lm + j)}; },
+        nl, cnt, [&](uint32_t j) { return NbrXL{V.cur.xs[j], V.lm[j]}; },
         [&](uint32_t j, const NbrXL& r) { one(j, r.x, r.lq); });
   }
 #ifndef PF_EXACT_ROUNDING
@@ -578,7 +581,7 @@ __global__ void k_s_xsph(WorldView V, uint32_t rank, uint32_t sub) {
   const uint32_t cnt = V.ncount[k];
   const NbrList nl = nbr_list(V, k);
   prefetch_list(nl, cnt);
-  const float* __restrict__ q_of = reinterpret_cast<const float*>(V.lm) + 1;  // lm[j].y: volume if > 0
+  const float* q_of = reinterpret_cast<const float*>(V.lm) + 1;  // lm[j].y: volume if > 0
   // without boundaries in the world every neighbour has the fluid volume
   auto one = [&](float4 xj, float4 vj, float bvj) {
     const f3 off = xi - xyz(xj);
@@ -596,7 +599,7 @@ __global__ void k_s_xsph(WorldView V, uint32_t rank, uint32_t sub) {
   };
   walk_nbrs<kNbrUnroll>(
       nl, cnt,
-      [&](uint32_t j) { return NbrXV{__ldg(V.cur.x + j), __ldg(V.cur.v + j), kBnd ? __ldg(q_of + 2 * (size_t)j) : 0.0f}; },
+      [&](uint32_t j) { return NbrXV{V.cur.x[j], V.cur.v[j], kBnd ? q_of[2 * (size_t)j] : 0.0f}; },
       [&](uint32_t, const NbrXV& r) { one(r.x, r.v, r.q); });
 #ifndef PF_EXACT_ROUNDING
   sm = sm * F.poly6;
@@ -629,7 +632,7 @@ __global__ void k_s_vort_grad(WorldView V, uint32_t rank, uint32_t sub) {
   prefetch_list(nl, cnt);
   walk_nbrs<kNbrUnroll>(
       nl, cnt,
-      [&](uint32_t j) { return NbrXV{__ldg(V.cur.x + j), V.vort[j], kBnd ? __ldg(V.cur.bv + j) : 0.0f}; },
+      [&](uint32_t j) { return NbrXV{V.cur.x[j], V.vort[j], kBnd ? V.cur.bv[j] : 0.0f}; },
       [&](uint32_t, const NbrXV& r) {
         if (kBnd && r.q > 0.0f) return;
         const f3 off = xi - xyz(r.x);
@@ -658,7 +661,7 @@ __global__ void k_s_color_normal(WorldView V, uint32_t rank, uint32_t sub) {
   const NbrList nl = nbr_list(V, k);
   prefetch_list(nl, cnt);
   walk_nbrs<kNbrUnroll>(
-      nl, cnt, [&](uint32_t j) { return NbrXQ{__ldg(V.cur.xs + j), kBnd ? __ldg(V.cur.bv + j) : 0.0f}; },
+      nl, cnt, [&](uint32_t j) { return NbrXQ{V.cur.xs[j], kBnd ? V.cur.bv[j] : 0.0f}; },
       [&](uint32_t, const NbrXQ& r) {
         const f3 off = xi - xyz(r.x);
         sum = sum + spiky_vec(off, dot(off, off), F) * (kBnd && r.q > 0.0f ? r.q : F.volume);
@@ -745,10 +748,10 @@ __global__ void k_s_impulses(WorldView V, uint32_t rank, uint32_t sub) {
         nl, cnt,
         [&](uint32_t j) {
           NbrXN r;
-          r.x = __ldg(V.cur.xs + j);
+          r.x = V.cur.xs[j];
           r.n = st ? V.normal[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          r.q = ad ? __ldg(V.cur.bv + j) : 0.0f;
-          r.tag = homog ? f : __ldg(V.cur.tag + j);
+          r.q = ad ? V.cur.bv[j] : 0.0f;
+          r.tag = homog ? f : V.cur.tag[j];
           return r;
         },
         [&](uint32_t j, const NbrXN& n) {
@@ -765,7 +768,7 @@ __global__ void k_s_impulses(WorldView V, uint32_t rank, uint32_t sub) {
   const uint32_t idi = V.ids[k];
   for (uint32_t m = 0; m < cnt; ++m) {
     const uint32_t j = nl.entry(m);
-    const f3 off = xi - xyz(__ldg(V.cur.xs + j));
+    const f3 off = xi - xyz(V.cur.xs[j]);
     if (st) {
       const uint32_t idj = V.ids[j];
       if (idj > idi && idj < F.range_end) {
@@ -778,7 +781,7 @@ __global__ void k_s_impulses(WorldView V, uint32_t rank, uint32_t sub) {
       }
     }
     if (ad) {
-      const float vol = __ldg(V.cur.bv + j);
+      const float vol = V.cur.bv[j];
       if (vol > 0.0f) {
         const float r = len(off);
         if (!(r < 1e-20f)) acc_add(V.acc_imp, k, adhesion_change(F, off, r, vol, dt), F.imp_scale);

@@ -29,8 +29,8 @@ constexpr uint32_t kTileWarps = 4;     // warps (independent tiles) per CTA
 constexpr uint32_t kTileThreads = 32 * kTileWarps;
 
 // Halo rows of a tile: 9 rows in (dz, dy) order over cells [xa, xb].
-__device__ __forceinline__ void tile_rows(const DevScene& S, const uint32_t* __restrict__ cstart,
-                                          const uint32_t* __restrict__ ccount, int32_t y, int32_t z, int32_t x0,
+__device__ __forceinline__ void tile_rows(const DevScene& S, const uint32_t* cstart, const uint32_t* ccount,
+                                          int32_t y, int32_t z, int32_t x0,
                                           int32_t x1, uint32_t rs[9], uint32_t len[9]) {
   const int32_t xa = max(x0 - 1, 0), xb = min(x1 + 1, (int32_t)S.dims[0] - 1);
   int r = 0;
@@ -52,8 +52,8 @@ __device__ __forceinline__ void tile_rows(const DevScene& S, const uint32_t* __r
 // Next tile of a row starting at cell x (>= one occupied cell): at most
 // kTileMax particles and kTileCells cells, shrunk until its halo fits in a
 // warp's shared memory (a single cell always forms a tile).
-__device__ __forceinline__ int32_t next_tile(const DevScene& S, const uint32_t* __restrict__ cstart,
-                                            const uint32_t* __restrict__ ccount, uint32_t rowk, int32_t y, int32_t z,
+__device__ __forceinline__ int32_t next_tile(const DevScene& S, const uint32_t* cstart, const uint32_t* ccount,
+                                            uint32_t rowk, int32_t y, int32_t z,
                                             int32_t x0, uint32_t rs[9], uint32_t len[9], uint32_t* halo) {
   const int32_t nx = (int32_t)S.dims[0];
   int32_t x = x0;
@@ -184,7 +184,7 @@ __device__ __forceinline__ WarpTile load_warp_tile(const Tile* tiles, uint32_t t
 // Stage a tile's halo of per-slot data into the warp's shared memory with
 // asynchronous copies, row by row (coalesced within a row).
 template <typename E>
-__device__ __forceinline__ void stage_rows(const WarpTile& W, const E* __restrict__ src, E* dst) {
+__device__ __forceinline__ void stage_rows(const WarpTile& W, const E* src, E* dst) {
   const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
   for (int r = 0; r < 9; ++r) {
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(kTileThreads) k_t_neighbors(WorldView V, uint3
           const int32_t yy = cy + dy, zz = cz + dz;
           if (yy < 0 || yy >= (int32_t)S.dims[1] || zz < 0 || zz >= (int32_t)S.dims[2]) continue;
           const uint32_t row = S.cell_base + S.dims[0] * ((uint32_t)yy + S.dims[1] * (uint32_t)zz);
-          const uint32_t a = __ldg(V.cstart + row + xa);
-          const uint32_t b = __ldg(V.cstart + row + xb) + __ldg(V.ccount + row + xb);
+          const uint32_t a = V.cstart[row + xa];
+          const uint32_t b = V.cstart[row + xb] + V.ccount[row + xb];
           const uint32_t base = T.roff[r] - T.rs[r];
           for (uint32_t j = a; j < b; ++j) {
             const uint32_t h = base + j;
