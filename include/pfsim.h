@@ -404,7 +404,10 @@ PF_API pf_status pf_contacts_read(pf_scene* scene, uint32_t* pairs, uint32_t cap
                                   uint32_t* stored);
 
 /* SimLoop.step(dt) (loop.ts:267-279): one frame of `substeps` substeps, dt in
- * seconds (a double, as the reference's JavaScript number). Asynchronous. */
+ * seconds (a double, as the reference's JavaScript number). Asynchronous: up
+ * to three steps are queued ahead of the GPU, fewer (the call waits for an
+ * earlier step) while the particles spread in a grid window that they nearly
+ * fill, so that the window grows before it is outgrown. */
 PF_API pf_status pf_step(pf_scene* scene, double dt);
 
 

@@ -2219,7 +2219,7 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   sort_scratch_carve(static_cast<char*>(arena_) + probe.off, n_, sort_cells, &sort_);
   radix_ = radix_plan(cells_);
   cells_cap_ = cell_room;
-  grow_prev_ext_.assign(3 * K, 0);
+  spread_.assign(K, GridSpread{});
   base_.scenes = base_.scenes_rw;
   base_.n = n_;
   base_.prim_stride = prim_stride_;
@@ -3275,6 +3275,56 @@ pf_status World::step(double dt) {
   return PF_OK;
 }
 
+// Takes the cell bounds of the newest step whose copy has landed (the ring
+// holds the last kBoundsRing steps; those still queued are skipped), after
+// waiting for step `wait_for`'s unless that is negative: each scene's spread
+// per axis, its growth per step since the look before, and the scene's pace,
+// the fastest growth of late (a tenth is forgotten per look).
+pf_status World::look_at_bounds(int64_t wait_for) {
+  if (wait_for >= 0) PF_CUDA(cudaEventSynchronize(ev_bounds_[wait_for % kBoundsRing]));
+  const uint64_t oldest = std::max(bounds_seen_, steps_done_ > kBoundsRing ? steps_done_ - kBoundsRing : 0);
+  uint64_t t = steps_done_;
+  for (; t > oldest; --t) {
+    const cudaError_t e = cudaEventQuery(ev_bounds_[(t - 1) % kBoundsRing]);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorNotReady) PF_CUDA(e);
+  }
+  if (t <= oldest) return PF_OK;  // none that was not looked at already
+  const int64_t since = bounds_seen_ ? (int64_t)(t - bounds_seen_) : 1;  // steps since the last look
+  bounds_seen_ = t;
+  const int32_t* seen = h_pinned_bbox_ + 6 * h_scenes_.size() * ((t - 1) % kBoundsRing);
+  for (uint32_t s = 0; s < h_scenes_.size(); ++s) {
+    if (!h_scenes_[s].has_grid) continue;
+    GridSpread& G = spread_[s];
+    G.pace *= 0.9f;
+    for (int a = 0; a < 3; ++a) {
+      const int64_t mn = seen[6 * s + a], mx = seen[6 * s + a + 3];
+      if (mn > mx) continue;  // no particle
+      const int64_t ext = mx - mn + 1, prev = G.prev[a];
+      G.lo[a] = mn;
+      G.rate[a] = prev > 0 ? (std::max<int64_t>(0, ext - prev) + since - 1) / since : 0;
+      G.prev[a] = G.ext[a] = ext;
+      G.pace = std::max(G.pace, (float)G.rate[a]);
+    }
+  }
+  return PF_OK;
+}
+
+// Whether a window could fill up in the steps that the bounds last looked at
+// do not cover (the one about to be queued included), if its particles spread
+// at twice their pace, and by a cell per step at least.
+bool World::windows_close() const {
+  const float ahead = (float)(steps_done_ + 1 - bounds_seen_);
+  for (uint32_t s = 0; s < h_scenes_.size(); ++s) {
+    const GridSpread& G = spread_[s];
+    if (!h_scenes_[s].has_grid || G.refused) continue;
+    const float reach = ahead * std::max(1.0f, 2.0f * G.pace);
+    for (int a = 0; a < 3; ++a)
+      if (G.ext[a] > 0 && reach > (float)((int64_t)h_scenes_[s].dims[a] - G.ext[a])) return true;
+  }
+  return false;
+}
+
 // Before a step: a grid scene whose particles' cell bounds (as the window
 // fit of the newest step whose bounds have arrived saw them) come within a
 // margin of its window's size on some axis gets a window twice their spread
@@ -3282,71 +3332,50 @@ pf_status World::step(double dt) {
 // grid is unbounded). The margin covers the spread's growth over the steps
 // from those bounds to the end of the one about to be queued, and one more.
 // Windows past 2^27 cells stay as they are (their keys clamp and flag).
+//
+// Queueing a step costs the host microseconds, so a caller that reads nothing
+// between steps runs ahead of the bounds, and a window could be outgrown, and
+// clamp, before they arrive. Where that could happen (windows_close) the host
+// waits, for the oldest missing bounds first, so that the GPU keeps the steps
+// queued behind them. A fluid that walls hold, or whose window has room,
+// queues as far ahead as the parameters allow; only one that spreads in a
+// close window waits for the step just queued.
 pf_status World::maybe_grow_windows() {
   if (!any_grid_ || steps_done_ == 0) return PF_OK;
-  // A recorded step costs the host microseconds, so a caller that reads
-  // nothing between steps runs ahead of the bounds, and a window that fits
-  // the particles closely would be outgrown, and clamp, before they arrive.
-  // A plain scene therefore waits for the step before's bounds while a window
-  // is less than twice its particles' spread, and else for those of the step
-  // before that one, which leaves the GPU a step to work on meanwhile.
-  if (lazy_graph_ && steps_done_ >= kGraphAfter) {
-    const uint64_t t = steps_done_ - (windows_tight_ ? 1 : 2);
-    if (t + 1 > bounds_seen_) PF_CUDA(cudaEventSynchronize(ev_bounds_[t % kBoundsRing]));
-  }
-  // the newest step whose bounds have landed (the ring holds the last
-  // kBoundsRing steps; one that is still queued is skipped, not waited for)
-  uint64_t seen_step = 0;
-  bool found = false;
-  const uint64_t oldest = steps_done_ > kBoundsRing ? steps_done_ - kBoundsRing : 0;
-  for (uint64_t t = steps_done_; t-- > oldest;) {
-    if (t + 1 <= bounds_seen_) break;  // looked at already
-    const cudaError_t e = cudaEventQuery(ev_bounds_[t % kBoundsRing]);
-    if (e == cudaSuccess) {
-      seen_step = t;
-      found = true;
-      break;
-    }
-    if (e != cudaErrorNotReady) PF_CUDA(e);
-  }
-  if (!found) return PF_OK;
+  const uint64_t seen_before = bounds_seen_;
+  // the first look is at the step before the last at the latest
+  PF_TRY(look_at_bounds(bounds_seen_ == 0 && steps_done_ >= 2 ? (int64_t)steps_done_ - 2 : -1));
+  while (bounds_seen_ && bounds_seen_ < steps_done_ && windows_close())
+    PF_TRY(look_at_bounds((int64_t)std::max(bounds_seen_, steps_done_ > kBoundsRing ? steps_done_ - kBoundsRing : 0)));
+  if (bounds_seen_ == seen_before) return PF_OK;
   // steps from those bounds to the end of the step about to be queued
-  const uint64_t ahead = steps_done_ - seen_step;
-  const uint64_t since = bounds_seen_ ? seen_step + 1 - bounds_seen_ : 1;  // steps since the last look
-  bounds_seen_ = seen_step + 1;
-  const int32_t* seen = h_pinned_bbox_ + 6 * h_scenes_.size() * (seen_step % kBoundsRing);
-  bool any = false, tight = false;
+  const int64_t ahead = (int64_t)(steps_done_ + 1 - bounds_seen_);
+  bool any = false;
   for (uint32_t s = 0; s < h_scenes_.size(); ++s) {
     DevScene& S = h_scenes_[s];
     if (!S.has_grid) continue;
-    const int32_t* b = seen + 6 * s;
+    GridSpread& G = spread_[s];
     int64_t lo[3], dims[3];
     bool grow = false;
     for (int a = 0; a < 3; ++a) {
-      const int64_t mn = b[a], mx = b[a + 3], d = S.dims[a];
+      const int64_t ext = G.ext[a], d = S.dims[a];
       lo[a] = S.lo0[a];
       dims[a] = d;
-      if (mn > mx) continue;  // no particle
       // within two cells of clamping, plus the spread's growth per step
       // over the steps from these bounds to the end of the next one, and
       // one step more; a fluid that walls hold stops growing there
-      const int64_t ext = mx - mn + 1;
-      tight = tight || 2 * ext + 8 > d;
-      int32_t& prev = grow_prev_ext_[3 * s + a];
-      const int64_t rate = prev > 0 ? (std::max<int64_t>(0, ext - prev) + (int64_t)since - 1) / (int64_t)since : 0;
-      prev = (int32_t)ext;
-      if (ext + (int64_t)(ahead + 1) * rate + 4 <= d) continue;
+      if (ext == 0 || ext + (ahead + 1) * G.rate[a] + 4 <= d) continue;
       dims[a] = std::max<int64_t>(d, 2 * ext + 8);
-      lo[a] = ((mn + mx) >> 1) - dims[a] / 2;
+      lo[a] = G.lo[a] + (ext - 1) / 2 - dims[a] / 2;
       grow = true;
     }
     if (!grow) continue;
     const uint64_t cells = (uint64_t)dims[0] * dims[1] * dims[2];
-    if (cells > (1ull << 27)) continue;
-    for (int a = 0; a < 3; ++a) grow_prev_ext_[3 * s + a] = 0;
-    bool fits = true;
+    bool fits = cells <= (1ull << 27);
     for (int a = 0; a < 3; ++a) fits = fits && lo[a] > INT32_MIN / 2 && lo[a] + dims[a] < INT32_MAX / 2;
+    G.refused = !fits;
     if (!fits) continue;
+    for (int a = 0; a < 3; ++a) G.prev[a] = 0;
     const float org[3] = {S.ox, S.oy, S.oz};
     double big = 0;
     for (int a = 0; a < 3; ++a) {
@@ -3359,7 +3388,6 @@ pf_status World::maybe_grow_windows() {
     S.prune_slack = f32(big * (1.0 / 65536.0) + 1e-9);
     any = true;
   }
-  windows_tight_ = tight;
   if (!any) return PF_OK;
   return relayout_grid();
 }

@@ -656,8 +656,7 @@ class World {
   int32_t* h_pinned_bbox_ = nullptr;  // kBoundsRing buffers of 6 words per scene
   cudaEvent_t ev_bounds_[kBoundsRing] = {};
   uint64_t steps_done_ = 0;
-  uint64_t bounds_seen_ = 0;  // steps_done_ of the last bounds looked at, plus one (0: none yet)
-  bool windows_tight_ = true;  // a window was less than twice its particles' spread in the bounds last seen
+  uint64_t bounds_seen_ = 0;  // steps whose bounds, or those of a later one, have been looked at
   // Per-step parameters go through a ring of kParamRing pinned staging
   // buffers, so the host can queue that many steps ahead; a buffer is
   // written again once the event of its last upload has passed.
@@ -669,9 +668,20 @@ class World {
   void* grid_arena_ = nullptr;  // cell arrays once the windows outgrow the arena's
   void* sort_arena_ = nullptr;  // sort scratch once the windows pass the cells it was carved for
   uint64_t cells_cap_ = 0;      // cells the current cell arrays and sort scratch hold
-  std::vector<int32_t> grow_prev_ext_;  // per scene and axis: the spread in cells at the last look
+  // Per scene, from the bounds last looked at: per axis the lowest cell and
+  // the spread in cells (0: not seen yet), its growth per step since the look
+  // before (`prev`: the spread then, 0 once the window has grown), and the
+  // fastest growth of late; `refused`: the window cannot grow any further.
+  struct GridSpread {
+    int64_t lo[3] = {}, ext[3] = {}, prev[3] = {}, rate[3] = {};
+    float pace = 0;
+    bool refused = false;
+  };
+  std::vector<GridSpread> spread_;
   uint32_t regrowths_ = 0;
   bool graphs_stale_ = false;  // the windows grew: capture the graphs again before launching one
+  pf_status look_at_bounds(int64_t wait_for);
+  bool windows_close() const;
   pf_status maybe_grow_windows();
   pf_status relayout_grid();
 
