@@ -3,7 +3,7 @@
 // Replaces the reference's 8-kernel HashGrid rebuild (src/core/hashGrid/
 // cellIndex.ts:113-170, sort.ts:72-192): the reference's histogram ->
 // exclusive scan -> scatter becomes, for B200,
-//   * up to 65,536 elements, everything after the keys in one launch of a
+//   * up to 65,536 elements, every pass after the keys in one launch of a
 //     16-block cluster (k_small_sort);
 //   * past that, keys with every radix pass's digit counts, from
 //     shared-memory histograms (one global atomic per digit per block), and
@@ -619,25 +619,34 @@ k_radix_scatter(const uint32_t* kin, const uint32_t* vin, uint32_t n, uint32_t* 
 }
 
 // ------------------------------------------------------------ small sort ----
-// A sort of at most 65,536 elements in one thread-block cluster: every
-// pass, and the scan of the cell counts where the cells are few, in one
-// launch. A pass of the kernels above is three or four launches of a few
-// microseconds each, however few the elements; here the blocks exchange their
+// A sort of at most 65,536 elements in one thread-block cluster: every pass
+// in one launch. A pass of the kernels above is three or four launches of a
+// few microseconds each, however few the elements; here the blocks exchange their
 // digit counts through distributed shared memory and meet at the hardware
 // cluster barrier. The elements stay in registers within a pass and go from
 // pass to pass through L2. Ranks as in k_radix_scatter: by ballots within a
 // warp, against the warp's histogram over its rounds, over the block's warps,
 // then over the blocks, so the sort is stable.
-// A sort of 20,011 particles (two passes, 65,536 cells) took 40 us as linked
-// launches and takes 25 so; the sorts of a 50,000-particle pile's step (three
-// passes) went from about 45 to 29 us each. Above 65,536 elements more SMs
-// than a cluster's are worth the launches.
+//
+// Whole sorts, us, as the launches above and with this one (each with its keys
+// and cell scan):
+//   elements        64   2,000   5,000  20,011  32,768  50,000  65,536
+//   4,096 cells   24.7    31.8    30.8    37.2    30.7    31.0    31.0
+//                 17.4    19.5    19.6    23.6    23.6    29.8    29.8
+//   262,144       33.0    43.2    43.2    51.7    41.1    43.1    41.1
+//                 21.5    25.6    25.7    30.3    31.6    40.0    40.0
+//   1,000,000     36.1    45.9    47.1    55.3    45.1    47.1    46.1
+//                 23.5    27.7    28.3    33.8    36.0    42.6    43.9
+// So the line lies at what the cluster's registers hold, where the two meet.
+// A dam break's step (two sorts) of 5,000 particles takes 349 and 322 us so,
+// of 40,000 387 and 379, of 60,000 418 and 414. The scan of the cell counts
+// stays k_scan's: in the cluster it took 1 to 2 us more at 4,096 cells, 4 to 8
+// at 262,144 and 30 at 1,000,000.
 constexpr uint32_t kSmallThreads = 1024;
 constexpr uint32_t kSmallWarps = kSmallThreads / 32;
 constexpr uint32_t kSmallItems = 4;      // elements per thread at most
 constexpr uint32_t kSmallBlocks = 16;    // blocks of the cluster (8 where 16 cannot be resident)
 constexpr uint32_t kSmallDigits = 256;   // passes of 8 bits at most
-constexpr uint64_t kSmallScan = 262144;  // cells scanned in the cluster at most (else k_scan follows)
 
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -657,14 +666,13 @@ __device__ __forceinline__ uint32_t cluster_load(const uint32_t* p, uint32_t ran
 template <uint32_t kItems>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, uint2* a, uint2* b, uint32_t* perm,
-             uint32_t* count, uint32_t* start, uint32_t cells, uint32_t scan, const uint32_t* over, uint32_t* over_to) {
+             uint32_t* count, const uint32_t* over, uint32_t* over_to) {
   pdl_begin();
   __shared__ uint16_t whist[kSmallWarps][kSmallDigits];  // per warp: its digit counts, then their offsets
   __shared__ uint32_t part[4][kSmallDigits], prior[4][kSmallDigits], whole[4][kSmallDigits];
   __shared__ uint32_t mine[kSmallDigits];   // this block's digit counts (read by the others)
   __shared__ uint32_t first[kSmallDigits];  // first output position of this block's elements of each digit
   __shared__ uint32_t s_warp[kSmallWarps];
-  __shared__ uint32_t total;                // of this block's cells (read by the others)
   uint32_t blocks, me;
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(blocks));
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(me));
@@ -673,7 +681,7 @@ k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, 
   const uint32_t base = (me * kSmallWarps + warp) * (32u * kItems) + lane;  // element i of the thread: base + 32 i
   const uint32_t d4 = tid & (kSmallDigits - 1u), quarter = tid / kSmallDigits;
   // exclusive sum of v over the block's threads
-  auto block_exclusive = [&](uint32_t v, uint32_t* sum) {
+  auto block_exclusive = [&](uint32_t v) {
     uint32_t x = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -689,10 +697,7 @@ k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, 
       const uint32_t y = __shfl_up_sync(0xffffffffu, wi, off);
       if (lane >= (uint32_t)off) wi += y;
     }
-    *sum = __shfl_sync(0xffffffffu, wi, 31);
-    const uint32_t before = __shfl_sync(0xffffffffu, wi - w, warp);
-    __syncthreads();  // s_warp is free again
-    return before + x - v;
+    return __shfl_sync(0xffffffffu, wi - w, warp) + x - v;
   };
   if (over_to && me == 0 && tid == 0) *over_to = *over;
   const uint2* in = nullptr;
@@ -765,9 +770,8 @@ k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, 
       prior[quarter][d4] = before;
       whole[quarter][d4] = all;
       __syncthreads();
-      uint32_t sum;
       const uint32_t own = tid < kSmallDigits ? whole[0][tid] + whole[1][tid] + whole[2][tid] + whole[3][tid] : 0u;
-      const uint32_t excl = block_exclusive(own, &sum);
+      const uint32_t excl = block_exclusive(own);
       if (tid < kSmallDigits) first[tid] = excl + prior[0][tid] + prior[1][tid] + prior[2][tid] + prior[3][tid];
     }
     __syncthreads();
@@ -784,35 +788,6 @@ k_small_sort(const uint32_t* keys, uint32_t n, uint32_t passes, uint32_t width, 
     cluster_sync();
     in = out;
   }
-  if (!scan) return;
-  // cell counts -> starts: a run of cells per block, 4 a thread and round
-  const uint32_t per = (div_up(cells, blocks) + 3u) & ~3u;
-  const uint32_t c0 = min(me * per, cells), c1 = min(c0 + per, cells);
-  uint32_t sum = 0, block_sum;
-  for (uint32_t c = c0 + tid; c < c1; c += kSmallThreads) sum += __ldcg(count + c);
-  (void)block_exclusive(sum, &block_sum);
-  if (tid == 0) total = block_sum;
-  cluster_sync();
-  uint32_t carry = 0;
-  {
-    const uint32_t t = lane < blocks && lane < me ? cluster_load(&total, lane) : 0u;
-    carry = __reduce_add_sync(0xffffffffu, t);
-  }
-  for (uint32_t cc = c0; cc < c1; cc += 4u * kSmallThreads) {
-    const uint32_t c = cc + 4u * tid;
-    uint32_t v[4];
-#pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) v[q] = c + q < c1 ? __ldcg(count + c + q) : 0u;
-    uint32_t round;
-    uint32_t at = carry + block_exclusive(v[0] + v[1] + v[2] + v[3], &round);
-#pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) {
-      if (c + q < c1) start[c + q] = at;
-      at += v[q];
-    }
-    carry += round;
-  }
-  cluster_sync();  // no block leaves while another may read its total
 }
 
 // A plan of no passes (one cell): the identity permutation.
@@ -1022,7 +997,8 @@ cudaError_t launch_scatter_as(const uint32_t* kin, const uint32_t* vin, uint32_t
   const uint32_t grid = std::min<uint32_t>(radix_tiles(n), blocks * (uint32_t)sm_count());
   const bool vec = (reinterpret_cast<uintptr_t>(kin) & 15u) == 0 &&
                    (kFirst || (reinterpret_cast<uintptr_t>(vin) & 15u) == 0);
-  launch_kernel(k_radix_scatter<kFirst, kLast, kBallot, kW>, grid, kOsThreads, smem, st, kin, vin, n, kout, vout, shift, plan.digits, s.tcount, s.csum, count, vec ? 1u : 0u);
+  launch_kernel(k_radix_scatter<kFirst, kLast, kBallot, kW>, grid, kOsThreads, smem, st, kin, vin, n, kout, vout, shift,
+                plan.digits, s.tcount, s.csum, count, vec ? 1u : 0u);
   return cudaGetLastError();
 }
 
@@ -1091,15 +1067,14 @@ uint32_t small_blocks_of() {
              ? kSmallBlocks
              : 8u;
 }
-cudaError_t launch_small_sort(const uint32_t* keys, uint32_t n, uint64_t C, const RadixPlan& plan, uint32_t* count,
-                              uint32_t* start, uint32_t* perm, uint32_t* overflow, const SortScratch& s,
-                              cudaStream_t st) {
-  const uint32_t blocks = small_blocks(), lanes = blocks * kSmallThreads, scan = C <= kSmallScan ? 1u : 0u;
+cudaError_t launch_small_sort(const uint32_t* keys, uint32_t n, const RadixPlan& plan, uint32_t* count,
+                              uint32_t* perm, uint32_t* overflow, const SortScratch& s, cudaStream_t st) {
+  const uint32_t blocks = small_blocks(), lanes = blocks * kSmallThreads;
   auto go = [&](auto kernel) {
     // the scratch holds va behind ka (vb behind kb): room for n pairs
     return launch_cluster(kernel, blocks, blocks, kSmallThreads, 0, st, keys, n, plan.passes, plan.width,
-                          reinterpret_cast<uint2*>(s.ka), reinterpret_cast<uint2*>(s.kb), perm, count, start,
-                          (uint32_t)C, scan, s.counters + kCounterOverflow, overflow);
+                          reinterpret_cast<uint2*>(s.ka), reinterpret_cast<uint2*>(s.kb), perm, count,
+                          s.counters + kCounterOverflow, overflow);
   };
   if (n <= lanes) return go(k_small_sort<1>);
   if (n <= 2 * lanes) return go(k_small_sort<2>);
@@ -1111,9 +1086,9 @@ bool small_sort(const RadixPlan& plan, uint32_t n) {
   return n > 0 && plan.passes > 0 && plan.digits <= kSmallDigits && n <= small_blocks() * kSmallThreads * kSmallItems;
 }
 
-uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n, uint64_t C) {
+uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n) {
   if (n == 0) return 1;                        // the start scan
-  if (small_sort(plan, n)) return C <= kSmallScan ? 1u : 2u;
+  if (small_sort(plan, n)) return 2;           // the cluster, start scan
   if (plan.passes == 0) return 3;              // identity, run counts, start scan
   // digit scan, per pass four (three when the tiles form one chunk), start scan
   const uint32_t per_pass = div_up(radix_tiles(n), kScanChunk) > 1 ? 4u : 3u;
@@ -1125,9 +1100,8 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
                              cudaStream_t st) {
   if (C == 0) return cudaSuccess;
   if (small_sort(plan, n)) {
-    if (cudaError_t e = launch_small_sort(keys, n, C, plan, count, start, perm, overflow, s, st); e != cudaSuccess)
-      return e;
-    return C <= kSmallScan ? cudaSuccess : launch_start_scan(count, start, C, s, st);
+    if (cudaError_t e = launch_small_sort(keys, n, plan, count, perm, overflow, s, st); e != cudaSuccess) return e;
+    return launch_start_scan(count, start, C, s, st);
   }
   if (n > 0) {
     const uint32_t tiles = radix_tiles(n);
@@ -1150,9 +1124,10 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
         uint32_t* vout = last ? perm : ((p & 1u) ? s.vb : s.va);
         const uint32_t shift = p * plan.width;
         launch_kernel(k_tile_counts, tiles, kCountThreads, 0, st, kin, n, shift, plan.digits, s.tcount,
-                                                       (first ? kvec : true) ? 1u : 0u);
+                      (first ? kvec : true) ? 1u : 0u);
         const uint32_t* first_pos = s.digit_count + p * kRadixMaxDigits;
-        launch_kernel(k_tile_scan_chunk, dim3(chunks, div_up(plan.digits, 256)), 256, 0, st, s.tcount, tiles, plan.digits, s.csum, chunks == 1 ? first_pos : nullptr);
+        launch_kernel(k_tile_scan_chunk, dim3(chunks, div_up(plan.digits, 256)), 256, 0, st, s.tcount, tiles,
+                      plan.digits, s.csum, chunks == 1 ? first_pos : nullptr);
         if (chunks > 1)
           launch_kernel(k_tile_scan_chunks, div_up(plan.digits, 8), 256, 0, st, s.csum, chunks, plan.digits, first_pos);
         cudaError_t e;

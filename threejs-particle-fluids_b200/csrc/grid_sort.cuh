@@ -1,18 +1,21 @@
 // grid_sort.cuh — stable counting sort of particle indices by cell key.
 //
 // Pipeline (launch_grid_sort after the keys and their digit counts exist):
-//   keys+digits  key of every element (or the caller's keys), and the count
-//                of every radix digit of every pass, from shared-memory
-//                histograms flushed once per block
+//   keys+digits  key of every element (or the caller's keys), and, past
+//                65,536 elements, the count of every radix digit of every
+//                pass, from shared-memory histograms flushed once per block
+//   small sort   up to 65,536 elements: all LSD radix passes and the cell
+//                counts in one thread-block cluster, and then the scan below
 //   digit scan   the counts of each pass turned into each digit's first
 //                output position
 //   passes       one LSD radix pass per 8 (or fewer; PFSIM_RADIX_BITS) key
 //                bits, each three steps: every tile of 4096 elements counts
 //                its digits; the tile counts are scanned per digit over the
 //                tiles; a persistent scatter ranks each tile's elements by
-//                digit in element order (warp-aggregated with
-//                __match_any_sync), copying the next tile into shared memory
-//                meanwhile, and writes them out digit run by digit run
+//                digit in element order (warp-aggregated, equal digits found
+//                by a ballot per digit bit), copying the next tile into
+//                shared memory meanwhile, and writes them out digit run by
+//                digit run
 //   runs         the last pass writes no keys: it counts every cell from its
 //                staged tiles, which are in key order (one atomic per run of
 //                equal keys in a warp)
@@ -106,8 +109,8 @@ cudaError_t launch_grid_sort(const uint32_t* keys, uint32_t n, uint64_t C, const
                              uint32_t* count, uint32_t* start, uint32_t* perm, uint32_t* overflow,
                              const SortScratch& s, cudaStream_t st);
 
-// Kernel launches of launch_grid_sort for a plan, element and cell count.
-uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n, uint64_t C);
+// Kernel launches of launch_grid_sort for a plan and element count.
+uint32_t grid_sort_launches(const RadixPlan& plan, uint32_t n);
 // Whether n elements are sorted in one cluster (after radix_prepare).
 bool small_sort(const RadixPlan& plan, uint32_t n);
 

@@ -2993,7 +2993,7 @@ void World::run_sort_and_permute(uint32_t parity, bool bbox_ready) {
   const DigitHist hist = digit_hist(radix_, sort_, n_);
   launch_kernel(k_keys, keys_grid(n_, cells_, kBlock), kBlock, 4ull * hist.passes * hist.digits, stream_, V, hist, cells_);
   launch_grid_sort(V.keys, n_, cells_, radix_, V.ccount, V.cstart, V.perm, nullptr, sort_, stream_);
-  t_launches += 1 + grid_sort_launches(radix_, n_, cells_);  // the keys, then the sort
+  t_launches += 1 + grid_sort_launches(radix_, n_);  // the keys, then the sort
   launch_slots(k_permute, n_, stream_, V);
 }
 
