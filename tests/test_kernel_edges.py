@@ -325,3 +325,34 @@ def test_boundary_volume_lanes(oracle, m, static):
     x, y = (w.readback(N.PF_FIELD_BOUNDARY_VOLUME)[nf:].astype(np.float64) for w in (a, o))
     assert (y > 0).all() and (np.abs(x - y) <= 64 * 2.0**-23 * y).all()
     a.close()
+
+
+@pytest.mark.parametrize("blocks", [0, 8])
+def test_sort_where_the_cluster_cannot_be_placed(blocks):
+    """A device that places no 16-block cluster takes one of 8 blocks (half the
+    elements at most), or none and the separate passes: the stable order on
+    both sides of every line, in a process of its own (the choice is made
+    once)."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import PKG
+
+    code = """
+import numpy as np
+from pfsim import hashgrid as H
+for n in (1, 8191, 8193, 16384, 16385, 32768, 32769, 65536, 65537):
+    for dims in ((16, 16, 1), (64, 64, 65)):
+        r = np.random.default_rng(n)
+        pos = np.zeros((n, 4), np.float32)
+        pos[:, :3] = r.uniform(0.0, 1.0, (n, 3)) * np.array(dims) * 0.1
+        pos[: n // 2, :3] = pos[n - 1, :3]
+        a = H.sort(pos, H.GridOptions(cell_size=0.1, kind="linear", dims=dims))
+        assert np.array_equal(a.sorted_indices, np.argsort(a.cell_index, kind="stable")), (n, dims)
+        count = np.bincount(a.cell_index, minlength=int(np.prod(dims)))
+        assert np.array_equal(a.counts, count) and np.array_equal(a.cell_start, np.cumsum(count) - count), (n, dims)
+"""
+    env = dict(os.environ, PYTHONPATH=str(PKG), PFSIM_SORT_CLUSTER=str(blocks))
+    p = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]

@@ -645,7 +645,7 @@ k_radix_scatter(const uint32_t* kin, const uint32_t* vin, uint32_t n, uint32_t* 
 constexpr uint32_t kSmallThreads = 1024;
 constexpr uint32_t kSmallWarps = kSmallThreads / 32;
 constexpr uint32_t kSmallItems = 4;      // elements per thread at most
-constexpr uint32_t kSmallBlocks = 16;    // blocks of the cluster (8 where 16 cannot be resident)
+constexpr uint32_t kSmallBlocks = 16;    // blocks of the cluster (8, or no cluster, where 16 cannot be resident)
 constexpr uint32_t kSmallDigits = 256;   // passes of 8 bits at most
 
 __device__ __forceinline__ void cluster_sync() {
@@ -1054,18 +1054,27 @@ cudaLaunchConfig_t small_config(uint32_t blocks, cudaStream_t st) {
   cfg.stream = st;
   return cfg;
 }
+// The largest of 16 and 8 blocks (up to PFSIM_SORT_CLUSTER) whose cluster
+// the device can place, else 0. A refused query leaves no error behind.
 template <uint32_t kItems>
 uint32_t small_blocks_of() {
-  if (cudaFuncSetAttribute(k_small_sort<kItems>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    return 8;
-  cudaLaunchAttribute at = cluster_attribute(kSmallBlocks);
-  cudaLaunchConfig_t cfg = small_config(kSmallBlocks, nullptr);
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  return cudaOccupancyMaxActiveClusters(&clusters, k_small_sort<kItems>, &cfg) == cudaSuccess && clusters > 0
-             ? kSmallBlocks
-             : 8u;
+  uint32_t most = kSmallBlocks;
+  if (const char* e = std::getenv("PFSIM_SORT_CLUSTER")) most = (uint32_t)std::atoi(e);  // for measurements and tests
+  for (uint32_t blocks = kSmallBlocks; blocks >= 8; blocks /= 2) {
+    if (blocks > most) continue;
+    cudaLaunchAttribute at = cluster_attribute(blocks);
+    cudaLaunchConfig_t cfg = small_config(blocks, nullptr);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    cudaError_t e = cudaSuccess;
+    if (blocks > 8)
+      e = cudaFuncSetAttribute(k_small_sort<kItems>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, k_small_sort<kItems>, &cfg);
+    if (e == cudaSuccess && clusters > 0) return blocks;
+    if (e != cudaSuccess) cudaGetLastError();
+  }
+  return 0;
 }
 cudaError_t launch_small_sort(const uint32_t* keys, uint32_t n, const RadixPlan& plan, uint32_t* count,
                               uint32_t* perm, uint32_t* overflow, const SortScratch& s, cudaStream_t st) {
@@ -1166,7 +1175,6 @@ cudaError_t radix_prepare() {
   if (dev < 64) g_smem_per_sm[dev] = per_sm;
   if (dev < 64)
     g_small_blocks[dev] = std::min({small_blocks_of<1>(), small_blocks_of<2>(), small_blocks_of<kSmallItems>()});
-  cudaGetLastError();
   (void)sm_count();  // cached outside any stream capture
   ready.insert(dev);
   return cudaSuccess;

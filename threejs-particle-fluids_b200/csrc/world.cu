@@ -2985,14 +2985,14 @@ void World::run_sort_and_permute(uint32_t parity, bool bbox_ready) {
   const WorldView V = view(parity);
   const uint32_t K = (uint32_t)h_scenes_.size();
   if (!bbox_ready) {
-    sort_state_zero(sort_, cells_, stream_);
+    note_launch(sort_state_zero(sort_, cells_, stream_));
     launch_slots(k_bbox, n_, stream_, V);
   }
   launch_kernel(k_grid_fit, div_up(K, 128), 128, 0, stream_, V, K);
   ++t_launches;
   const DigitHist hist = digit_hist(radix_, sort_, n_);
   launch_kernel(k_keys, keys_grid(n_, cells_, kBlock), kBlock, 4ull * hist.passes * hist.digits, stream_, V, hist, cells_);
-  launch_grid_sort(V.keys, n_, cells_, radix_, V.ccount, V.cstart, V.perm, nullptr, sort_, stream_);
+  note_launch(launch_grid_sort(V.keys, n_, cells_, radix_, V.ccount, V.cstart, V.perm, nullptr, sort_, stream_));
   t_launches += 1 + grid_sort_launches(radix_, n_);  // the keys, then the sort
   launch_slots(k_permute, n_, stream_, V);
 }
@@ -3034,7 +3034,7 @@ void World::launch_aero(const WorldView& V, uint32_t stage, uint32_t s) {
 
 void World::run_substep(uint32_t s, uint32_t parity) {
   WorldView V = view(parity);
-  if (any_grid_) sort_state_zero(sort_, cells_, stream_);
+  if (any_grid_) note_launch(sort_state_zero(sort_, cells_, stream_));
   launch_slots(k_predict, n_, stream_, V, s);
   if (any_soft_local_) launch_slots(k_rot_predict, base_.n_grp, stream_, V, s);
   if (any_grid_) {
@@ -3219,7 +3219,12 @@ pf_status World::step(double dt) {
       PF_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
       body(p);
       launches_per_step_ = t_launches;
+      const cudaError_t refused = take_launch_error();
       PF_CUDA(cudaStreamEndCapture(stream_, &graph));
+      if (refused != cudaSuccess) {  // a step without one of its launches is not kept
+        cudaGraphDestroy(graph);
+        PF_CUDA(refused);
+      }
       if (g) {
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(g, graph, &info) != cudaSuccess) {
@@ -3271,8 +3276,17 @@ pf_status World::step(double dt) {
     PF_CUDA(cudaEventRecord(ev_bounds_[q], stream_));
   }
   ++steps_done_;
-  PF_CUDA(cudaGetLastError());
+  PF_CUDA(take_launch_error());
   return PF_OK;
+}
+
+// The first error of the launches since the last call: those that returned
+// one (a sort takes its own from the runtime) or left one there.
+cudaError_t World::take_launch_error() {
+  note_launch(cudaGetLastError());
+  const cudaError_t e = launch_error_;
+  launch_error_ = cudaSuccess;
+  return e;
 }
 
 // Takes the cell bounds of the newest step whose copy has landed (the ring

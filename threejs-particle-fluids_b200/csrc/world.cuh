@@ -523,6 +523,11 @@ class World {
   // bbox_ready: the predict pass of this substep gathered the cell bounds
   // the grid window follows (otherwise a separate pass gathers them)
   void run_sort_and_permute(uint32_t parity, bool bbox_ready);
+  cudaError_t launch_error_ = cudaSuccess;
+  void note_launch(cudaError_t e) {
+    if (launch_error_ == cudaSuccess) launch_error_ = e;
+  }
+  cudaError_t take_launch_error();
   void run_init_pass();
   void launch_tiles_build(const WorldView& V, uint32_t s);
   template <typename K, typename... A>
