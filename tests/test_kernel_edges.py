@@ -356,3 +356,48 @@ for n in (1, 8191, 8193, 16384, 16385, 32768, 32769, 65536, 65537):
     env = dict(os.environ, PYTHONPATH=str(PKG), PFSIM_SORT_CLUSTER=str(blocks))
     p = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr[-2000:]
+
+
+def _lattice_body(k, offset, spin):
+    """A k^3 lattice of 2 cm spacing with edges between near points, spinning."""
+    g = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3) * 0.02
+    d = np.abs(g[:, None] - g[None]).max(-1)
+    e = np.argwhere((d < 0.025) & (np.arange(len(g))[:, None] < np.arange(len(g))[None]))
+    return (g + offset).astype(np.float32), np.cross(spin, g - g.mean(0)).astype(np.float32), e.astype(np.uint32)
+
+
+def _chain_edges(n):
+    return np.stack([np.arange(n - 1), np.arange(1, n)], 1).astype(np.uint32)
+
+
+def test_softbodies_of_a_batch_at_different_ranks(pfsim):
+    """Scenes whose soft bodies are their first and their second material, in
+    one batch: the positions, orientations and so the spins of the scenes
+    stepped alone."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    recs = []
+    for fluid_first in (False, True):
+        x, v, e = _lattice_body(4, [0.3, 0.4, 0.3], np.array([8.0, -5.0, 3.0]))
+        ups, mats = [R.Upload(0, x, v, np.full(64, 125.0, np.float32))], []
+        soft = ("soft", R.SoftbodyOpts([R.BodyDef(range=(0, 64), compliance=1e-5, edges=_chain_edges(64))], "local"))
+        if fluid_first:
+            f = (np.random.default_rng(4).uniform(0, 0.1, (200, 3)) + [0.6, 0.05, 0.3]).astype(np.float32)
+            ups.append(R.Upload(64, f))
+            mats.append(("fluid", R.FluidOpts(range=(64, 200), particle_spacing=0.02, rest_density=1000.0,
+                                              viscosity=0.01)))
+        mats.append(soft)
+        recs.append(R.Recipe(capacity=264 if fluid_first else 64, radius=0.01, uploads=ups, materials=mats,
+                             prims=R.container_walls((0.0, 0.0, 0.0), (1.0, 1.0, 1.0)),
+                             loop=R.LoopOpts(substeps=2, iterations=2)))
+    alone = [R.NativeBackend().build(r) for r in recs]
+    batch = R.Batch([R.NativeBackend().build(r) for r in recs])
+    for _ in range(3):
+        batch.step(1 / 60)
+        for s in alone:
+            s.step(1 / 60)
+    for i, s in enumerate(alone):
+        for f in (N.PF_FIELD_POSITIONS, N.PF_FIELD_ROTATION):
+            assert np.array_equal(s.readback(f)[:64], batch.readback(i, f)[:64]), (i, f)
+    batch.close()

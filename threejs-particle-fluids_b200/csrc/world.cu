@@ -766,14 +766,15 @@ __global__ void __launch_bounds__(kBlock) k_rot_predict(WorldView V, uint32_t su
   V.qp[i] = with_w(nx, ch * q.w - dot(sx, qx));
 }
 
-// rotation.ts:316-343
-__global__ void __launch_bounds__(kBlock) k_rot_advect(WorldView V, uint32_t sub) {
+// rotation.ts:316-343, for the systems that are their scene's material `rank`
+// (once a substep each: a second time would find no turn, and stop the spin).
+__global__ void __launch_bounds__(kBlock) k_rot_advect(WorldView V, uint32_t rank, uint32_t sub) {
   pdl_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= V.n_grp) return;
   const DevSoft& D = V.softs[V.grp_soft[g]];
   const DevScene& S = V.scenes[D.scene];
-  if (sub >= S.substeps) return;
+  if (D.rank != rank || sub >= S.substeps) return;
   const uint32_t i = V.grp[g];
   const float4 q = V.q[i];
   float4 qp = V.qp[i];
@@ -3150,7 +3151,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
       launch_slots(k_xsph_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s);
     }
     if (has_local) {
-      launch_slots(k_rot_advect, base_.n_grp, stream_, V, s);
+      launch_slots(k_rot_advect, base_.n_grp, stream_, V, r, s);
       if (base_.n_bodies) {
         launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, 0u, 0u);
         ++t_launches;
