@@ -370,6 +370,54 @@ def _chain_edges(n):
     return np.stack([np.arange(n - 1), np.arange(1, n)], 1).astype(np.uint32)
 
 
+@pytest.mark.parametrize("second", ["local", "global"])
+@pytest.mark.parametrize("case", ["apart", "around", "around_reversed", "shared", "part_shared"])
+def test_two_softbody_systems(oracle, case, second):
+    """Two soft-body systems in one scene: one after the other, one whose
+    bodies lie on both sides of the other's, and over the same particles (all
+    or some of them) with clusters and rest shapes of their own: the oracle's
+    positions and orientations after two frames."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    spin = np.array([6.0, -9.0, 4.0])
+    parts = [_lattice_body(k, [0.2 + 0.25 * b, 0.4, 0.3], spin) for b, k in enumerate((3, 4, 3))]
+    first = np.cumsum([0] + [len(p[0]) for p in parts])
+    pos, vel = np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
+    n = len(pos)
+
+    def body(b, edges=None, scale=1.0, compliance=1e-5):
+        rest = parts[b][0] * np.float32(scale)
+        return R.BodyDef(range=(int(first[b]), len(parts[b][0])), compliance=compliance, rest_positions=rest,
+                         edges=parts[b][2] if edges is None else edges)
+
+    if case == "apart":
+        a, b = [body(0)], [body(1), body(2)]
+    elif case.startswith("around"):
+        a, b = [body(0), body(2)], [body(1)]
+    elif case == "shared":
+        a, b = [body(0), body(1)], [body(0, _chain_edges(27), 1.02, 1e-4), body(1, scale=0.99)]
+    else:
+        a, b = [body(0), body(1)], [body(1, _chain_edges(64), 1.01, 1e-4), body(2)]
+    mats = [("soft", R.SoftbodyOpts(a, "local")), ("soft", R.SoftbodyOpts(b, second))]
+    if case == "around_reversed":
+        mats.reverse()
+    rec = R.Recipe(capacity=n, radius=0.01, uploads=[R.Upload(0, pos, vel, np.full(n, 125.0, np.float32))],
+                   materials=mats, prims=R.container_walls((0.0, 0.0, 0.0), (1.0, 1.0, 1.0)),
+                   loop=R.LoopOpts(substeps=2, iterations=3))
+    s, o = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    for _ in range(2):
+        s.step(1 / 60)
+        o.step(1 / 60)
+    # positions within 1e-5 of the container's metre a frame; quaternions of
+    # unit length, from rotations of clusters a few centimetres wide
+    x, y = s.readback(N.PF_FIELD_POSITIONS), o.readback(N.PF_FIELD_POSITIONS)
+    assert np.abs(x - y).max() <= 2e-5
+    q, p = s.readback(N.PF_FIELD_ROTATION), o.readback(N.PF_FIELD_ROTATION)
+    assert np.abs(q - p).max() <= 1e-3
+    s.close()
+
+
 def test_softbodies_of_a_batch_at_different_ranks(pfsim):
     """Scenes whose soft bodies are their first and their second material, in
     one batch: the positions, orientations and so the spins of the scenes

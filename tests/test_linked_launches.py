@@ -17,7 +17,7 @@ LINKED = ["grid_sort.cu", "grid_sort.cuh", "world.cu", "world_contacts.cuh", "wo
 # and the members of shape-matching clusters.
 TABLES = {
     "world_kernels.cuh": {"list": "chunk_slot", "b": "sdf_trilinear", "V.plane4": None},
-    "world.cu": {"w": "stage_prims", "V.mem_info": None, "V.mem": None},
+    "world.cu": {"w": "stage_prims", "V.mem_info": None, "V.mem": None, "V.mem_soft": None},
 }
 
 

@@ -977,10 +977,9 @@ __global__ void __launch_bounds__(kSmBlock, 8) k_sm_gather(WorldView V, uint32_t
     // do not depend on them), so the chains of dependent loads overlap
     M = __ldg(V.mem_info + t / L);  // id, first entry, entries, members of its own cluster
     j = M.x;
-    const uint32_t soft = V.mem_soft[j];
+    D = &V.softs[__ldg(V.mem_soft + t / L)];
     sj = V.inv[j];
     rest4 = V.rest[j];
-    D = &V.softs[soft];
     xj = V.cur.xs[sj];
     S = &V.scenes[D->scene];
     act = D->rank == rank && sub < S->substeps && it < S->iterations;
@@ -1028,25 +1027,12 @@ __global__ void __launch_bounds__(kSmBlock, 8) k_sm_gather(WorldView V, uint32_t
   }
   // the cluster centred on the particle takes its quaternion (no lane reads
   // one in this pass; k_sm_moment's is the next to)
-  if (V.sm_qp_by_member && act && lane == L - 1 && M.w > 0) cluster_quaternion(V, j);
+  if (act && lane == L - 1) cluster_quaternion(V, j);
   if (!act || lane != 0 || !(tx | ty | tz)) return;
   bool sat = false;
   const f3 ch = ticks_change((int)tx, (int)ty, (int)tz, S->sb_inv, &sat);
   V.cur.xs[sj] = with_w(xyz(xj) + ch, xj.w);
   if (sat) atomicOr(V.flags + D->scene * kNumFlags + FLAG_SOFT, 1u);
-}
-
-// Cluster quaternions whose particle is in no cluster of its own system (no
-// lane of k_sm_gather stands for it).
-__global__ void __launch_bounds__(kBlock) k_sm_qp(WorldView V, uint32_t rank, uint32_t sub, uint32_t it) {
-  pdl_begin();
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= V.n_grp) return;
-  const DevSoft* D;
-  const DevScene* S;
-  if (!group_active(V, g, rank, sub, it, &D, &S)) return;
-  const uint32_t i = V.grp[g];
-  if (V.csr_off[i + 1] > V.csr_off[i]) cluster_quaternion(V, i);
 }
 
 // shapeMatch.ts:53-229: one 256-thread block per body reduces the centre of
@@ -1886,72 +1872,100 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     damp_ranges_[r] = {begin, (uint32_t)dvtx.size()};
   }
   // ---- soft-body tables (global by id) ----------------------------------
-  std::vector<uint32_t> grp, grp_soft, csr_off(n_ + 1, 0), csr_idx;
-  std::vector<float> rest4(4ull * n_, 0.0f), restc4(4ull * n_, 0.0f), weights(n_, 0.0f);
+  // per system: its groups (one per particle of its span, a cluster each in
+  // local systems) and the clusters' members, as a CSR over the groups.
+  // The rest shapes of a rank's systems go to the first layer where no rank
+  // before has bodies of the same particles.
+  std::vector<uint32_t> grp, grp_soft, csr_off(1, 0), csr_idx;
+  std::vector<std::pair<uint32_t, uint32_t>> local_groups;  // per local system: first group, particle of it
+  size_t n_layers = 1;
+  uint64_t entries = 0;
+  std::vector<float> rest4, restc4, weights;
+  soft_layer_.assign(max_rank_, 0);
   {
+    std::vector<std::vector<std::vector<RangeU>>> taken;  // per layer and scene: the bodies on it
+    for (uint32_t r = 0; r < max_rank_; ++r) {
+      size_t layer = 0;
+      auto soft_of = [&](uint32_t s) -> const SoftSpec* {
+        const SceneSpec& sp = *specs[s];
+        const bool soft = r < sp.materials.size() && sp.materials[r].first == MAT_SOFT;
+        return soft ? &sp.softs[sp.materials[r].second] : nullptr;
+      };
+      auto free_on = [&](size_t l) {
+        for (uint32_t s = 0; s < K; ++s)
+          if (const SoftSpec* ss = soft_of(s))
+            for (const RangeU& t : taken[l][s])
+              for (const BodySpec& b : ss->bodies)
+                if (t.start < b.range.start + b.range.count && b.range.start < t.start + t.count) return false;
+        return true;
+      };
+      while (layer < taken.size() && !free_on(layer)) ++layer;
+      for (uint32_t s = 0; s < K; ++s)
+        if (const SoftSpec* ss = soft_of(s)) {
+          if (layer == taken.size()) taken.resize(layer + 1, std::vector<std::vector<RangeU>>(K));
+          for (const BodySpec& b : ss->bodies) taken[layer][s].push_back(b.range);
+          soft_layer_[r] = (uint32_t)layer;
+          n_layers = std::max(n_layers, layer + 1);
+          if (ss->local) entries += ss->offsets[ss->span.start + ss->span.count] - ss->offsets[ss->span.start];
+        }
+    }
+    if (entries > 0xffffffffull) return fail(PF_ERR_INVALID, "SoftbodySystem: too many cluster members");
+    csr_idx.reserve(entries);
+    if (!h_softs_.empty()) {
+      rest4.assign(4ull * n_ * n_layers, 0.0f);
+      restc4.assign(4ull * n_ * n_layers, 0.0f);
+      weights.assign((size_t)n_ * n_layers, 0.0f);
+    }
     uint32_t di = 0;
-    std::vector<uint32_t> deg(n_, 0);
-    std::vector<std::pair<uint32_t, const SoftSpec*>> locals;  // (scene, spec)
     for (uint32_t s = 0; s < K; ++s) {
       const SceneSpec& sp = *specs[s];
       const uint32_t base = h_scenes_[s].seg_start;
       for (uint32_t r = 0; r < sp.materials.size(); ++r) {
         if (sp.materials[r].first != MAT_SOFT) continue;
         const SoftSpec& ss = sp.softs[sp.materials[r].second];
-        for (uint32_t i = 0; i < sp.cap; ++i) {
-          if (ss.weights[i] != 0.0f || ss.rest4[4 * i + 3] != 0.0f || ss.rest4[4 * i] != 0.0f ||
-              ss.rest4[4 * i + 1] != 0.0f || ss.rest4[4 * i + 2] != 0.0f) {
-            for (int c = 0; c < 4; ++c) rest4[4ull * (base + i) + c] = ss.rest4[4 * i + c];
-            weights[base + i] = ss.weights[i];
+        const size_t at = (size_t)n_ * soft_layer_[r] + base;
+        for (const BodySpec& b : ss.bodies)
+          for (uint32_t i = b.range.start; i < b.range.start + b.range.count; ++i) {
+            for (int c = 0; c < 4; ++c) rest4[4 * (at + i) + c] = ss.rest4[4 * i + c];
+            weights[at + i] = ss.weights[i];
+            if (ss.local)
+              for (int c = 0; c < 4; ++c) restc4[4 * (at + i) + c] = ss.rest_centers4[4 * i + c];
           }
-        }
         if (ss.local) {
+          local_groups.push_back({(uint32_t)grp.size(), base + ss.span.start});
           for (uint32_t i = ss.span.start; i < ss.span.start + ss.span.count; ++i) {
             grp.push_back(base + i);
             grp_soft.push_back(di);
-            deg[base + i] = ss.offsets[i + 1] - ss.offsets[i];
-            for (int c = 0; c < 4; ++c) restc4[4ull * (base + i) + c] = ss.rest_centers4[4 * i + c];
+            for (uint32_t k = ss.offsets[i]; k < ss.offsets[i + 1]; ++k) csr_idx.push_back(base + ss.indices[k]);
+            csr_off.push_back((uint32_t)csr_idx.size());
           }
-          locals.push_back({s, &ss});
         }
         ++di;
       }
     }
-    for (uint32_t i = 0; i < n_; ++i) csr_off[i + 1] = csr_off[i] + deg[i];
-    csr_idx.assign(std::max<uint32_t>(1, csr_off[n_]), 0);
-    for (auto& [s, ss] : locals) {
-      const uint32_t base = h_scenes_[s].seg_start;
-      for (uint32_t i = ss->span.start; i < ss->span.start + ss->span.count; ++i) {
-        const uint32_t from = ss->offsets[i], to = ss->offsets[i + 1];
-        for (uint32_t k = from; k < to; ++k) csr_idx[csr_off[base + i] + (k - from)] = base + ss->indices[k];
-      }
-    }
   }
-  // the clusters that hold each particle (their centre ids) by member
-  std::vector<uint32_t> mem_off(n_ + 1, 0), mem_soft(n_, 0), mem_ids;
+  // the clusters that hold each particle (their centre ids) by member of a
+  // system: a member is found by its group there
+  std::vector<uint32_t> mem_off(grp.size() + 1, 0), mem_soft;
   std::vector<uint32_t> mem;
   std::vector<uint4> mem_info;
   // the moment pass's clusters, and their members' ids: by warp of clusters,
   // entry m of its 32 clusters side by side where that pads them to at most
-  // about twice their members, else cluster after cluster
+  // about twice their members (and the entries stay countable), else cluster
+  // after cluster
   std::vector<uint4> sm_grp(grp.size());
   std::vector<uint32_t> sm_ids;
   for (size_t w = 0; w < grp.size(); w += 32) {
     const size_t e = std::min(grp.size(), w + 32);
-    uint64_t most = 0, all = 0;
-    for (size_t g = w; g < e; ++g) {
-      const uint32_t deg = csr_off[grp[g] + 1] - csr_off[grp[g]];
-      most = std::max<uint64_t>(most, deg);
-      all += deg;
-    }
-    const bool side = 32 * most <= 2 * all + 256;
+    uint64_t most = 0;
+    for (size_t g = w; g < e; ++g) most = std::max<uint64_t>(most, csr_off[g + 1] - csr_off[g]);
+    const uint64_t all = csr_off[e] - csr_off[w], later = csr_off[grp.size()] - csr_off[e];
     const size_t base = sm_ids.size();
-    if (base + std::max(32 * most, all) > 0xffffffffull)
-      return fail(PF_ERR_INVALID, "SoftbodySystem: too many cluster members");
+    const bool side = 32 * most <= 2 * all + 256 && base + 32 * most + later <= 0xffffffffull;
     sm_ids.resize(base + (side ? 32 * most : all), grp[w]);
     size_t at = base;
     for (size_t g = w; g < e; ++g) {
-      const uint32_t from = csr_off[grp[g]], deg = csr_off[grp[g] + 1] - from;
+      const uint32_t from = csr_off[g], deg = csr_off[g + 1] - from;
       const size_t first = side ? base + (g - w) : at;
       const uint32_t stride = side ? 32u : 1u;
       for (uint32_t m = 0; m < deg; ++m) sm_ids[first + (size_t)m * stride] = csr_idx[from + m];
@@ -1959,20 +1973,25 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       at += deg;
     }
   }
-  bool qp_by_member = true;
   {
-    for (uint32_t g = 0; g < grp.size(); ++g)
-      for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) {
-        ++mem_off[csr_idx[m] + 1];
-        mem_soft[csr_idx[m]] = grp_soft[g];
+    // the group of a member of cluster g: its system's groups are in a row
+    std::vector<uint32_t> member(csr_idx.size());
+    for (size_t q = 0; q < local_groups.size(); ++q) {
+      const uint32_t g0 = local_groups[q].first, id0 = local_groups[q].second;
+      const uint32_t g1 = q + 1 < local_groups.size() ? local_groups[q + 1].first : (uint32_t)grp.size();
+      for (uint32_t m = csr_off[g0]; m < csr_off[g1]; ++m) {
+        member[m] = g0 + (csr_idx[m] - id0);
+        ++mem_off[member[m] + 1];
       }
+    }
     std::vector<uint32_t> held;  // clusters holding each member
-    for (uint32_t i = 0; i < n_; ++i) {
-      if (mem_off[i + 1]) {
-        mem_ids.push_back(i);
-        held.push_back(mem_off[i + 1]);
-      }
-      mem_off[i + 1] += mem_off[i];
+    for (uint32_t g = 0; g < grp.size(); ++g) {
+      const uint32_t n = mem_off[g + 1];
+      mem_off[g + 1] += mem_off[g];
+      if (!n) continue;
+      held.push_back(n);
+      mem_info.push_back(make_uint4(grp[g], mem_off[g], n, csr_off[g + 1] - csr_off[g]));
+      mem_soft.push_back(grp_soft[g]);
     }
     // lanes per member in k_sm_gather: the smallest power of two that takes
     // the clusters of nine members in ten in at most sixteen rounds (two for
@@ -1993,18 +2012,10 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       const uint32_t l = (uint32_t)std::atoi(e);
       if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) mem_lanes_ = l;
     }
-    for (uint32_t g = 0; g < grp.size(); ++g)
-      if (csr_off[grp[g] + 1] > csr_off[grp[g]])
-        qp_by_member = qp_by_member && mem_off[grp[g] + 1] > mem_off[grp[g]] && mem_soft[grp[g]] == grp_soft[g];
-    mem_info.resize(mem_ids.size());
-    mem.assign(mem_off[n_], 0u);
-    for (size_t t = 0; t < mem_ids.size(); ++t) {
-      const uint32_t id = mem_ids[t];
-      mem_info[t] = make_uint4(id, mem_off[id], mem_off[id + 1] - mem_off[id], csr_off[id + 1] - csr_off[id]);
-    }
+    mem.assign(csr_idx.size(), 0u);
     std::vector<uint32_t> at(mem_off.begin(), mem_off.end() - 1);
     for (uint32_t g = 0; g < grp.size(); ++g)
-      for (uint32_t m = csr_off[grp[g]]; m < csr_off[grp[g] + 1]; ++m) mem[at[csr_idx[m]]++] = grp[g];
+      for (uint32_t m = csr_off[g]; m < csr_off[g + 1]; ++m) mem[at[member[m]]++] = grp[g];
   }
   // ---- chunk table and per-slot state ----------------------------------
   std::vector<uint32_t> chunk(n_ / kSegAlign, 0);
@@ -2137,10 +2148,9 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     base_.bodies = cv.take<DevBody>(h_bodies_.size());
     base_.grp = cv.take<uint32_t>(grp.size());
     base_.grp_soft = cv.take<uint32_t>(grp_soft.size());
-    base_.csr_off = need_soft ? cv.take<uint32_t>(N + 1) : nullptr;
-    base_.rest = need_soft ? cv.take<float4>(N) : nullptr;
-    base_.rest_c = need_soft ? cv.take<float4>(N) : nullptr;
-    base_.weights = need_soft ? cv.take<float>(N) : nullptr;
+    base_.rest = need_soft ? cv.take<float4>(n_layers * N) : nullptr;
+    base_.rest_c = need_soft ? cv.take<float4>(n_layers * N) : nullptr;
+    base_.weights = need_soft ? cv.take<float>(n_layers * N) : nullptr;
     base_.rot4 = need_soft ? cv.take<float4>(4 * N) : nullptr;
     base_.q = need_soft ? cv.take<float4>(N) : nullptr;
     base_.qp = need_soft ? cv.take<float4>(N) : nullptr;
@@ -2150,10 +2160,10 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
     base_.sm_grp = cv.take<uint4>(sm_grp.size());
     base_.sm_ids = cv.take<uint32_t>(sm_ids.size());
     base_.sm_slots = any_grid_ ? cv.take<uint32_t>(sm_ids.size()) : const_cast<uint32_t*>(base_.sm_ids);
-    base_.mem_soft = any_soft_local_ ? cv.take<uint32_t>(N) : nullptr;
+    base_.mem_soft = any_soft_local_ ? cv.take<uint32_t>(mem_soft.size()) : nullptr;
     base_.mem_info = any_soft_local_ ? cv.take<uint4>(mem_info.size()) : nullptr;
-    base_.n_mem_ids = any_soft_local_ ? (uint32_t)mem_ids.size() : 0u;
-    base_.lambda_g = need_soft ? cv.take<float4>(N) : nullptr;
+    base_.n_mem_ids = any_soft_local_ ? (uint32_t)mem_info.size() : 0u;
+    base_.lambda_g = need_soft ? cv.take<float4>(n_layers * N) : nullptr;
     base_.body_c = cv.take<float4>(h_bodies_.size());
     base_.body_r = cv.take<float4>(3 * h_bodies_.size());
     base_.c_i = cv.take<uint32_t>(ci.size());
@@ -2226,7 +2236,6 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   base_.prim_stride = prim_stride_;
   base_.n_grp = (uint32_t)grp.size();
   base_.n_sm = (uint32_t)sm_ids.size();
-  base_.sm_qp_by_member = qp_by_member ? 1u : 0u;
   base_.n_bodies = (uint32_t)h_bodies_.size();
   base_.n_cons = (uint32_t)ci.size();
   base_.n_bend = (uint32_t)bidx.size();
@@ -2328,7 +2337,6 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   PF_TRY(up(base_.grp, grp.data(), 4 * grp.size()));
   PF_TRY(up(base_.grp_soft, grp_soft.data(), 4 * grp_soft.size()));
   if (need_soft) {
-    PF_TRY(up(base_.csr_off, csr_off.data(), 4 * csr_off.size()));
     if (any_soft_local_) {
       PF_TRY(up(base_.mem, mem.data(), 4 * mem.size()));
       PF_TRY(up(base_.sm_grp, sm_grp.data(), sizeof(uint4) * sm_grp.size()));
@@ -2336,9 +2344,9 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
       PF_TRY(up(const_cast<uint32_t*>(base_.mem_soft), mem_soft.data(), 4 * mem_soft.size()));
       PF_TRY(up(base_.mem_info, mem_info.data(), sizeof(uint4) * mem_info.size()));
     }
-    PF_TRY(up(base_.rest, rest4.data(), 16 * N));
-    PF_TRY(up(base_.rest_c, restc4.data(), 16 * N));
-    PF_TRY(up(base_.weights, weights.data(), 4 * N));
+    PF_TRY(up(base_.rest, rest4.data(), 4 * rest4.size()));
+    PF_TRY(up(base_.rest_c, restc4.data(), 4 * restc4.size()));
+    PF_TRY(up(base_.weights, weights.data(), 4 * weights.size()));
     std::vector<float4> ident(3 * h_bodies_.size());
     for (size_t b = 0; b < h_bodies_.size(); ++b) {
       ident[3 * b] = make_float4(1, 0, 0, 0);
@@ -2638,6 +2646,17 @@ WorldView World::group_view(const WorldView& V, size_t g) const {
   W.fchunk = base_.fchunk + groups_[g].first;
   W.n_fchunk = groups_[g].second - groups_[g].first;
   return W;
+}
+
+// The rest shapes of rank `r`'s soft bodies.
+WorldView World::soft_view(const WorldView& V, uint32_t r) const {
+  WorldView R = V;
+  const size_t at = (size_t)soft_layer_[r] * n_;
+  R.rest += at;
+  R.rest_c += at;
+  R.weights += at;
+  R.lambda_g += at;
+  return R;
 }
 
 WorldView World::rest_view(const WorldView& V) const {
@@ -3107,24 +3126,24 @@ void World::run_substep(uint32_t s, uint32_t parity) {
         for (auto& S : h_scenes_) rest = rest || (S.fluid_count && !S.homog);
         if (rest) launch_slots(k_fluid_apply, VF.n_fchunk * kSegAlign, stream_, VF, r, s, it, slot ? 1u : 0u);
       }
+      const WorldView VS = has_local || has_global ? soft_view(V, r) : V;
       if (has_local) {
-        launch_kernel(k_sm_moment, div_up(base_.n_grp, kSmBlock), kSmBlock, 0, stream_, V, r, s, it);
+        launch_kernel(k_sm_moment, div_up(base_.n_grp, kSmBlock), kSmBlock, 0, stream_, VS, r, s, it);
         ++t_launches;
         if (base_.n_mem_ids) {  // mem_lanes_ lanes per cluster member
           const uint32_t grid = (uint32_t)(((uint64_t)mem_lanes_ * base_.n_mem_ids + kSmBlock - 1) / kSmBlock);
-          if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kSmBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 2) launch_kernel(k_sm_gather<2>, grid, kSmBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 4) launch_kernel(k_sm_gather<4>, grid, kSmBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 8) launch_kernel(k_sm_gather<8>, grid, kSmBlock, 0, stream_, V, r, s, it);
-          else if (mem_lanes_ == 16) launch_kernel(k_sm_gather<16>, grid, kSmBlock, 0, stream_, V, r, s, it);
-          else launch_kernel(k_sm_gather<32>, grid, kSmBlock, 0, stream_, V, r, s, it);
+          if (mem_lanes_ == 1) launch_kernel(k_sm_gather<1>, grid, kSmBlock, 0, stream_, VS, r, s, it);
+          else if (mem_lanes_ == 2) launch_kernel(k_sm_gather<2>, grid, kSmBlock, 0, stream_, VS, r, s, it);
+          else if (mem_lanes_ == 4) launch_kernel(k_sm_gather<4>, grid, kSmBlock, 0, stream_, VS, r, s, it);
+          else if (mem_lanes_ == 8) launch_kernel(k_sm_gather<8>, grid, kSmBlock, 0, stream_, VS, r, s, it);
+          else if (mem_lanes_ == 16) launch_kernel(k_sm_gather<16>, grid, kSmBlock, 0, stream_, VS, r, s, it);
+          else launch_kernel(k_sm_gather<32>, grid, kSmBlock, 0, stream_, VS, r, s, it);
           ++t_launches;
         }
-        if (!base_.sm_qp_by_member) launch_slots(k_sm_qp, base_.n_grp, stream_, V, r, s, it);
       }
       if (has_global && base_.n_bodies) {
-        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, it, 1u);
-        launch_kernel(k_global_apply, base_.n_bodies, 256, 0, stream_, V, r, s, it);
+        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, VS, r, s, it, 1u);
+        launch_kernel(k_global_apply, base_.n_bodies, 256, 0, stream_, VS, r, s, it);
         t_launches += 2;
       }
       if (!fork && r < cloth_ranges_.size()) launch_cloth_rank(V, r, s, it, stream_);
@@ -3153,7 +3172,7 @@ void World::run_substep(uint32_t s, uint32_t parity) {
     if (has_local) {
       launch_slots(k_rot_advect, base_.n_grp, stream_, V, r, s);
       if (base_.n_bodies) {
-        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, V, r, s, 0u, 0u);
+        launch_kernel(k_body_frame, base_.n_bodies, 256, 0, stream_, soft_view(V, r), r, s, 0u, 0u);
         ++t_launches;
       }
     }

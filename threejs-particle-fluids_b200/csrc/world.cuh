@@ -348,7 +348,7 @@ struct WorldView {
   const uint32_t* grp;       // group ids (local shape matching)
   const uint32_t* grp_soft;  // soft index per group
   uint32_t n_grp;
-  const uint32_t* csr_off;   // by id, n + 1
+  // by id, the layer of the rank that a launch is for (soft_view)
   const float4* rest;        // rest offsets, w = compliance
   const float4* rest_c;      // neighbourhood rest centres
   const float* weights;
@@ -360,9 +360,10 @@ struct WorldView {
   float4* qp;                // predicted orientation
   float4* omega;             // angular velocity
   float4* pair_lambda;       // per entry of mem
-  // the clusters that hold each particle: per member (ascending ids) its id,
-  // first entry and entries of mem (the clusters' centre ids), and the members
-  // of its own cluster; mem_soft[j] is particle j's soft system
+  // the clusters that hold each particle: per member of a system (system by
+  // system, ascending ids) its id, first entry and entries of mem (the
+  // clusters' centre ids), and the members of its own cluster; mem_soft: its
+  // soft system
   const uint4* mem_info;
   const uint32_t* mem;
   const uint32_t* mem_soft;
@@ -372,9 +373,8 @@ struct WorldView {
   const uint32_t* sm_ids;
   uint32_t* sm_slots;
   uint32_t n_sm;
-  uint32_t sm_qp_by_member;  // every cluster's particle is a member: k_sm_gather takes the quaternions
   uint32_t n_mem_ids;
-  float4* lambda_g;          // global matching multipliers per id
+  float4* lambda_g;          // global matching multipliers, by id, of the rank's layer
   float4* body_c;            // per body
   float4* body_r;            // 3 rows per body
   uint32_t n_bodies;
@@ -543,6 +543,8 @@ class World {
   void run_groups(const WorldView& V, uint32_t s, bool apply);
   WorldView group_view(const WorldView& V, size_t g) const;
   WorldView rest_view(const WorldView& V) const;  // the other fluid scenes' chunks
+  WorldView soft_view(const WorldView& V, uint32_t r) const;
+  std::vector<uint32_t> soft_layer_;  // per rank: the layer of its soft bodies' rest shapes
   void apply_grouping();  // groups_ and the scenes' grouped flags from tune_.group
   bool grouping() const { return tune_.path == 0 && !groups_.empty(); }
   pf_status tune();
