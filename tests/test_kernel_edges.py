@@ -449,3 +449,101 @@ def test_softbodies_of_a_batch_at_different_ranks(pfsim):
         for f in (N.PF_FIELD_POSITIONS, N.PF_FIELD_ROTATION):
             assert np.array_equal(s.readback(f)[:64], batch.readback(i, f)[:64]), (i, f)
     batch.close()
+
+
+def _two_fluids_on_one_slab(a_bnd, b_bnd):
+    """Two fluids side by side on a slab of free particles, each with its own
+    range of the slab as a dynamic boundary."""
+    from pfsim import recipe as R
+
+    s = 0.02
+    fluid = np.stack(np.meshgrid(np.arange(4), np.arange(4), np.arange(8), indexing="ij"), -1).reshape(-1, 3) * s
+    slab = np.stack(np.meshgrid(np.arange(8), np.arange(2), np.arange(8), indexing="ij"), -1).reshape(-1, 3) * s
+    r = np.random.default_rng(11)
+    pos = np.concatenate([fluid + [0.3, 0.34, 0.3], fluid + [0.38, 0.34, 0.3], slab + [0.3, 0.3, 0.3]])
+    pos = (pos + r.uniform(-0.1 * s, 0.1 * s, pos.shape)).astype(np.float32)
+    opts = dict(particle_spacing=s, smoothing_radius=2 * s, rest_density=1000.0, viscosity=0.01)
+    mats = [("fluid", R.FluidOpts(range=(128 * k, 128), boundaries=[(256 + b, n) for b, n in bnd],
+                                  boundary_static=[False] * len(bnd), **opts)) for k, bnd in enumerate((a_bnd, b_bnd))]
+    return R.Recipe(capacity=384, radius=0.01, uploads=[R.Upload(0, pos, None, np.full(384, 125.0, np.float32))],
+                    materials=mats, prims=R.container_walls((0.0, 0.0, 0.0), (1.0, 1.0, 1.0)),
+                    loop=R.LoopOpts(substeps=2, iterations=3))
+
+
+@pytest.mark.parametrize("b_bnd", [[(32, 96)], [(64, 64), (0, 48)], []])
+@pytest.mark.parametrize("a_bnd", [[(0, 96)], [(16, 16), (40, 60)]])
+def test_reactions_on_a_boundary_of_two_fluids(oracle, nbr_path, a_bnd, b_bnd):
+    """Slab particles on one fluid's boundary, on both fluids' (their tag
+    names the second fluid's, so the first one's ranges are searched), and on
+    none: the oracle's positions within 1e-5 of the box, from reactions that
+    move the slab by much more than that."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    rec = _two_fluids_on_one_slab(a_bnd, b_bnd)
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend().build(rec)
+    a.step(1 / 60)
+    b.step(1 / 60)
+    x, y = a.readback(N.PF_FIELD_POSITIONS), b.readback(N.PF_FIELD_POSITIONS)
+    assert np.abs(x - y).max() <= 1e-5
+    a.close()
+
+
+@pytest.mark.parametrize("kind", ["pile", "cloth", "mixed", "surface"])
+def test_recorded_steps_of_every_material_same_bits(pfsim, monkeypatch, kind):
+    """Plain scenes through the step that records their graphs and several
+    recorded ones, with a dt that changes every frame: the bits of the same
+    scenes stepped without graphs, for contacts, shape matching, a full cloth,
+    fluid with soft bodies and a moving collider, and surface effects."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+    from pfsim import workloads as W
+
+    monkeypatch.setenv("PFSIM_NBR_PATH", "0")  # the autotuner could pick another path for each
+    if kind == "pile":
+        rec = W.softbody_pile(6000, seed=2, per_body=300)
+        rec.loop.contact = True
+    elif kind == "cloth":
+        rec = W.cloth_sheet(40, seed=3, bend_compliance=1e-5, tethers=True, stretch_tolerance=0.06,
+                            wind=(0.8, 0.0, 1.5), damping=0.2)
+    elif kind == "mixed":
+        rec = W.mixed_scene(6000, 4000, 4, seed=4)
+    else:
+        rec = W.dam_break(3000, seed=5)
+        o = rec.materials[0][1]
+        o.surface_tension, o.vorticity = 0.05, 0.02
+    a = R.NativeBackend().build(rec)
+    b = R.Batch([R.NativeBackend().build(rec)], use_graph=False)
+    for k in range(9):
+        dt = (1 / 60, 1 / 75, 1 / 50)[k % 3]
+        a.step(dt)
+        b.step(dt)
+        for f in (N.PF_FIELD_POSITIONS, N.PF_FIELD_VELOCITIES):
+            assert np.array_equal(a.readback(f), b.readback(0, f)), k
+    a.close()
+    b.close()
+
+
+def test_recorded_steps_follow_a_moved_sdf_collider(oracle):
+    """An SDF sphere that starts to move once the steps are recorded, under
+    particles that rest on it and fall past it: the oracle's positions within
+    1e-5 of the metre they stand in, frame by frame."""
+    from pfsim import _native as N
+    from pfsim import recipe as R
+
+    r = np.random.default_rng(9)
+    pos = np.concatenate([r.uniform(-0.2, 0.2, (60, 1)), r.uniform(0.26, 0.6, (60, 1)),
+                          r.uniform(-0.2, 0.2, (60, 1))], 1).astype(np.float32)
+    rec = R.Recipe(capacity=60, radius=0.01, uploads=[R.Upload(0, pos, None, np.full(60, 100.0, np.float32))],
+                   sdfs=[R.sphere_sdf((0.0, 0.0, 0.0), 0.25)], loop=R.LoopOpts(substeps=2, iterations=2))
+    a, b = R.NativeBackend().build(rec), oracle.OracleBackend(precision=32).build(rec)
+    for k in range(12):
+        if k >= 5:
+            at, q = (C.c_float * 3)(0.01 * (k - 4), 0.02 * (k - 4), 0.0), (C.c_float * 4)(0.0, 0.0, 0.0, 1.0)
+            N.check(N.lib().pf_set_sdf_transform(a.h, 0, at, q, 1.0))
+            oracle.check(oracle.lib().or_set_sdf_transform(b.h, 0, at, q, 1.0))
+        a.step(1 / 60)
+        b.step(1 / 60)
+        x, y = a.readback(N.PF_FIELD_POSITIONS), b.readback(N.PF_FIELD_POSITIONS)
+        assert np.abs(x - y).max() <= 1e-5, k
+    a.close()
