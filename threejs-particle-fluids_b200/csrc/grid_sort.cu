@@ -958,15 +958,16 @@ cudaError_t sort_state_zero(const SortScratch& s, uint64_t C, cudaStream_t st) {
 void launch_keys_digits(const float4* pos, uint32_t n, const KeyFn& kf, const RadixPlan& plan, uint32_t* keys,
                         uint32_t* overflow, uint32_t* count, uint64_t C, const SortScratch& s, cudaStream_t st) {
   const DigitHist h = digit_hist(plan, s, n);
-  launch_kernel(k_keys_digits, keys_grid(n, C, kHistThreads), kHistThreads, 4ull * h.passes * h.digits, st, pos, n, kf, h, keys,
-                overflow, count, C);
+  launch_kernel(k_keys_digits, keys_grid(n, C, kHistThreads), kHistThreads, 4ull * h.passes * h.digits, st, pos, n, kf, h,
+                keys, overflow, count, C);
 }
 
 namespace {
 // Cell counts -> cell starts (its tile status and ticket zeroed before).
 cudaError_t launch_start_scan(const uint32_t* in, uint32_t* out, uint64_t n, const SortScratch& s, cudaStream_t st) {
   const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-  return launch_kernel(k_scan, scan_tiles(n), kScanThreads, 0, st, in, out, n, s.scan_status, s.counters, vec ? 1u : 0u);
+  return launch_kernel(k_scan, scan_tiles(n), kScanThreads, 0, st, in, out, n, s.scan_status, s.counters,
+                       vec ? 1u : 0u);
 }
 }  // namespace
 

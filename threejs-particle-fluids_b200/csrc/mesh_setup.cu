@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(32 * kBakeWarps, 8) k_bake(const MeshTri* __re
       const TriCull& C = culls[t];
       const float far = square(gap(sx.lo, sx.hi, C.lo[0], C.hi[0]), gap(sy.lo, sy.hi, C.lo[1], C.hi[1]),
                                gap(sz.lo, sz.hi, C.lo[2], C.hi[2]));
-      const float off = fmaxf(fabsf(C.n[0] * fx + C.n[1] * fy + C.n[2] * fz - C.d) - (fuzz + C.slack), 0.0f) * 0.999999f;
+      const float off =
+          fmaxf(fabsf(C.n[0] * fx + C.n[1] * fy + C.n[2] * fz - C.d) - (fuzz + C.slack), 0.0f) * 0.999999f;
       if (far > best_up || off * off > best_up) continue;  // no closer than the best so far
       const double d = point_tri_d2(px, py, pz, tris[t]);
       if (d < best) {
@@ -780,11 +781,12 @@ pf_status pf_bake_sdf(const pf_mesh* mesh, uint32_t resolution, double padding, 
   PF_CUDA(dd.alloc(4 * n));
   PF_CUDA(dc.alloc(8));
   PF_CUDA(cudaMemset(dc.p, 0, 8));
-  const uint64_t bricks = (uint64_t)div_up(resolution, kBrickX) * div_up(resolution, kBrickY) * div_up(resolution, kBrickZ);
+  const uint64_t bricks =
+      (uint64_t)div_up(resolution, kBrickX) * div_up(resolution, kBrickY) * div_up(resolution, kBrickZ);
   k_bake<<<(unsigned)((bricks + kBakeWarps - 1) / kBakeWarps), 32 * kBakeWarps>>>(
       static_cast<const MeshTri*>(dt.p), static_cast<const TriCull*>(dk.p), (uint32_t)tris.size(),
-      static_cast<const ChunkBox*>(db.p), (uint32_t)boxes.size(), resolution, origin[0], origin[1], origin[2], vs, vs * 1e-4, static_cast<float*>(dd.p),
-      static_cast<unsigned long long*>(dc.p));
+      static_cast<const ChunkBox*>(db.p), (uint32_t)boxes.size(), resolution, origin[0], origin[1], origin[2], vs,
+      vs * 1e-4, static_cast<float*>(dd.p), static_cast<unsigned long long*>(dc.p));
   PF_TRY(occupancy_launch_check());
   PF_CUDA(cudaMemcpy(data, dd.p, 4 * n, cudaMemcpyDeviceToHost));
   unsigned long long bad = 0;

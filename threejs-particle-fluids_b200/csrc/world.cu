@@ -508,8 +508,8 @@ __global__ void __launch_bounds__(kBlock) k_friction(WorldView V, uint32_t sub) 
 // ---------------------------------------------------------------- cloth ----
 constexpr int kClothBlock = 128;
 // distance.ts:264-288 for one colour of constraints (no two share a particle).
-__global__ void __launch_bounds__(kClothBlock) k_cloth(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it,
-                                                  bool early) {
+__global__ void __launch_bounds__(kClothBlock) k_cloth(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
+                                                       uint32_t it, bool early) {
   if (!early) pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   bool act = q < end;
@@ -550,8 +550,8 @@ __global__ void __launch_bounds__(kClothBlock) k_cloth(WorldView V, uint32_t beg
 // theta = atan2((N1 x N2).E, (N1.N2)|E|) with E = p2 - p1,
 // N1 = (p3 - p1) x (p3 - p2), N2 = (p4 - p2) x (p4 - p1), and the XPBD
 // multiplier update (xpbd.ts:26-36).
-__global__ void __launch_bounds__(kClothBlock) k_bend(WorldView V, uint32_t begin, uint32_t end, uint32_t sub, uint32_t it,
-                                                 bool early) {
+__global__ void __launch_bounds__(kClothBlock) k_bend(WorldView V, uint32_t begin, uint32_t end, uint32_t sub,
+                                                      uint32_t it, bool early) {
   if (!early) pdl_begin();
   const uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x;
   bool act = q < end;
@@ -3011,7 +3011,8 @@ void World::run_sort_and_permute(uint32_t parity, bool bbox_ready) {
   launch_kernel(k_grid_fit, div_up(K, 128), 128, 0, stream_, V, K);
   ++t_launches;
   const DigitHist hist = digit_hist(radix_, sort_, n_);
-  launch_kernel(k_keys, keys_grid(n_, cells_, kBlock), kBlock, 4ull * hist.passes * hist.digits, stream_, V, hist, cells_);
+  launch_kernel(k_keys, keys_grid(n_, cells_, kBlock), kBlock, 4ull * hist.passes * hist.digits, stream_, V, hist,
+                cells_);
   note_launch(launch_grid_sort(V.keys, n_, cells_, radix_, V.ccount, V.cstart, V.perm, nullptr, sort_, stream_));
   t_launches += 1 + grid_sort_launches(radix_, n_);  // the keys, then the sort
   launch_slots(k_permute, n_, stream_, V);
@@ -3698,8 +3699,8 @@ pf_status World::import_scene(uint32_t s, const World& src, uint32_t src_s) {
   if (S.cap == 0) return PF_OK;
   const StateBuf& B = src.buf_[src.parity_];
   const WorldView V = view(parity_);
-  launch_kernel(k_import_scene, div_up(S.cap, kBlock), kBlock, 0, stream_, V, S.seg_start, S.cap, B.x, B.v, B.bv, src.base_.inv,
-                                                                 T.seg_start, src.base_.q, src.base_.omega);
+  launch_kernel(k_import_scene, div_up(S.cap, kBlock), kBlock, 0, stream_, V, S.seg_start, S.cap, B.x, B.v, B.bv,
+                src.base_.inv, T.seg_start, src.base_.q, src.base_.omega);
   PF_CUDA(cudaGetLastError());
   return PF_OK;
 }

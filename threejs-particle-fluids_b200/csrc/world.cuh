@@ -627,7 +627,6 @@ class World {
   bool lazy_graph_ = false;
   cudaGraphExec_t graph_[2] = {nullptr, nullptr};
   void drop_graphs();
-  double graph_dt_ = -1;
   cudaStream_t stream_ = nullptr;
   // second stream for cloth-only scenes (fork/join inside each substep)
   bool side_ok_ = false;

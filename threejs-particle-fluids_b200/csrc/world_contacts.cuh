@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(kConBlock) k_con_gen(WorldView V, uint32_t sub
   uint32_t keep = 0;
 #pragma unroll
   for (int r = kRow0; r < 9; ++r)
-    if (jd[r] < lim && (rs[r] + lane > k || (kQuiet && V.cquiet[jd[r]])) && (gi == 0u || gi != V.cgroup[jd[r]])) keep |= 1u << r;
+    if (jd[r] < lim && (rs[r] + lane > k || (kQuiet && V.cquiet[jd[r]])) && (gi == 0u || gi != V.cgroup[jd[r]]))
+      keep |= 1u << r;
   uint32_t cnt = 0;
   const auto append = [&](bool hit, uint32_t j) {
     const uint32_t b = (__ballot_sync(0xffffffffu, hit) >> shift) & ((1u << kConLanes) - 1u);
