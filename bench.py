@@ -128,10 +128,10 @@ class SortWorkload:
     # of dram__bytes_read.sum + dram__bytes_write.sum over a sort's launches
     # from a one-pass ncu capture:
     #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,
-    #       dram__bytes_write.sum --clock-control none -s 40 -c 60 --csv
+    #       dram__bytes_write.sum --clock-control none -s 45 -c 60 --csv
     #       python bench.py --workload sort --steps 3 --warmup 3
     #       --no-cpu-baseline
-    TRAFFIC_PER_PARTICLE = 63.4
+    TRAFFIC_PER_PARTICLE = 63.9
 
     def launches(self) -> int:
         """Kernel launches of one sort: keys with digit counts, digit starts,
@@ -287,11 +287,11 @@ class BatchWorkload:
     #       dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
     #       -k regex:k_s_ -c 44 --csv python bench.py --steps 20 --warmup 3
     #       --no-cpu-baseline --no-plain --no-serve
-    # (PFSIM_NBR_WIDE=0 or 1 fixes the list entry width the autotuner would
-    # pick, for the figures of the other width). Keyed by that width in bits.
+    # Keyed by the list entry width in bits; for the width that the autotuner
+    # does not pick, the last field of its PFSIM_TUNE_CACHE line was changed.
     STAGE_TRAFFIC_PER_PARTICLE: dict[int, dict[int, float]] = {
-        16: {0: 151.1, 1: 127.6, 2: 168.9, 3: 140.0},
-        32: {0: 286.6, 1: 207.6, 2: 248.8, 3: 216.1},
+        16: {0: 123.8, 1: 127.7, 2: 168.8, 3: 140.0},
+        32: {0: 237.2, 1: 207.7, 2: 248.9, 3: 216.1},
     }
 
     def __init__(self, n_scenes: int = 256):

@@ -616,13 +616,15 @@ class World {
   // graph
   bool use_graph_ = false;
   // A plain scene's steps become a CUDA graph once it has taken kGraphAfter
-  // of them: a step is 65 to 320 launches of a few microseconds, which the
-  // host issues more slowly than the GPU runs them, while a capture costs as
-  // much as a few steps, so a scene stepped only a few times does without
-  // one. Per step with its read, launched and as a graph: 5,000 fluid
-  // particles 521 and 426 us, 30,000 with surface effects (317 launches) 2.90
-  // and 2.38 ms, a 50,000-particle pile 1.95 and 1.69, a 256 x 256 cloth (196
-  // launches) 1.29 and 0.90. A serving loop's plain mode stays without graphs.
+  // of them. What that gains is the host's time: 45 to 220 launches a step
+  // take it 0.09 (5,000 fluid particles), 0.20 (a 50,000-particle pile) to
+  // 0.40 ms (30,000 particles with surface effects), a recorded step 0.01 to
+  // 0.02, so 256 scenes stepped side by side take 27.8 ms a frame (33.0
+  // launched). A single awaited scene takes as long either way, now that its
+  // launches are linked (before, 30,000 particles with surface effects 2.90 ms
+  // launched and 2.38 recorded). A capture costs 0.3 to 0.9 ms, so a scene
+  // stepped only a few times does without one, and so does a serving loop's
+  // plain mode.
   static constexpr uint64_t kGraphAfter = 3;
   bool lazy_graph_ = false;
   cudaGraphExec_t graph_[2] = {nullptr, nullptr};
