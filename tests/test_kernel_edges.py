@@ -547,3 +547,36 @@ def test_recorded_steps_follow_a_moved_sdf_collider(oracle):
         x, y = a.readback(N.PF_FIELD_POSITIONS), b.readback(N.PF_FIELD_POSITIONS)
         assert np.abs(x - y).max() <= 1e-5, k
     a.close()
+
+
+def test_threads_read_one_scene_at_once(pfsim):
+    """Threads that read different fields of one scene at the same time, one
+    of them the whole batch's positions, get what one thread alone reads."""
+    from concurrent.futures import ThreadPoolExecutor
+    from threading import Barrier
+
+    from pfsim import _native as N
+    from pfsim import recipe as R
+    from pfsim import workloads as W
+
+    w = R.Batch([R.NativeBackend().build(W.dam_break(30000, seed=51))])
+    for _ in range(3):
+        w.step(1 / 60)
+
+    def positions():
+        out = np.empty((w.capacities[0], 4), np.float32)
+        N.check(N.lib().pf_batch_read_positions(w.h, out.ctypes.data_as(C.POINTER(C.c_float)), out.nbytes))
+        return out
+
+    fields = [N.PF_FIELD_POSITIONS, N.PF_FIELD_VELOCITIES, N.PF_FIELD_DENSITY, N.PF_FIELD_INV_MASS, N.PF_FIELD_LAMBDA]
+    reads = [lambda f=f: w.readback(0, f) for f in fields] + [positions]
+    alone = [r() for r in reads]
+    start = Barrier(len(reads))
+
+    def reader(k):
+        start.wait(60)
+        return sum(not np.array_equal(reads[k](), alone[k]) for _ in range(60))
+
+    with ThreadPoolExecutor(len(reads)) as pool:
+        assert list(pool.map(reader, range(len(reads)))) == [0] * len(reads)
+    w.close()

@@ -3570,13 +3570,15 @@ pf_status World::readback(uint32_t scene, uint32_t field, void* dst, size_t byte
   };
   auto rows = [&](const float4* src) -> pf_status {
     PF_TRY(need(16ull * cap));
-    PF_TRY(wait_reads());  // an async read may still copy out of stage_pos_
+    std::lock_guard<std::mutex> lock(read_mutex_);
+    PF_TRY(wait_staged());  // an async read may still copy out of stage_pos_
     launch_slots(k_gather_rows, cap, stream_, inv, cap, src, stage_pos_);
     return fetch(16ull * cap);
   };
   auto words = [&](const void* src, uint32_t width, uint32_t word, bool fluid_only) -> pf_status {
     PF_TRY(need(4ull * cap));
-    PF_TRY(wait_reads());
+    std::lock_guard<std::mutex> lock(read_mutex_);
+    PF_TRY(wait_staged());
     launch_slots(k_gather_words, cap, stream_, inv, cap, static_cast<const float*>(src), width, word,
                  fluid_only ? (const uint32_t*)B.tag : nullptr, reinterpret_cast<float*>(stage_pos_));
     return fetch(4ull * cap);
@@ -3811,7 +3813,8 @@ uint64_t World::total_particles() const {
 pf_status World::read_positions(float* dst, size_t bytes) {
   const uint64_t total = total_particles();
   if (bytes < 16ull * total) return fail(PF_ERR_INVALID, "readback: destination too small");
-  PF_TRY(wait_reads());  // an async read may still copy out of stage_pos_
+  std::lock_guard<std::mutex> lock(read_mutex_);
+  PF_TRY(wait_staged());  // an async read may still copy out of stage_pos_
   launch_slots(k_gather_positions, n_, stream_, view(parity_), (const uint64_t*)prefix_dev_, stage_pos_);
   PF_CUDA(cudaMemcpyAsync(dst, stage_pos_, 16ull * total, cudaMemcpyDeviceToHost, stream_));
   PF_CUDA(cudaStreamSynchronize(stream_));
@@ -3821,6 +3824,7 @@ pf_status World::read_positions(float* dst, size_t bytes) {
 pf_status World::read_positions_async(float* dst, size_t bytes) {
   const uint64_t total = total_particles();
   if (bytes < 16ull * total) return fail(PF_ERR_INVALID, "readback: destination too small");
+  std::lock_guard<std::mutex> lock(read_mutex_);
   if (!read_stream_) {
     PF_CUDA(cudaStreamCreateWithFlags(&read_stream_, cudaStreamNonBlocking));
     for (int b = 0; b < 2; ++b) {
@@ -3845,6 +3849,11 @@ pf_status World::read_positions_async(float* dst, size_t bytes) {
 }
 
 pf_status World::wait_reads() {
+  std::lock_guard<std::mutex> lock(read_mutex_);
+  return wait_staged();
+}
+
+pf_status World::wait_staged() {
   for (int b = 0; b < 2; ++b)
     if (read_pending_[b]) {
       PF_CUDA(cudaEventSynchronize(ev_read_[b]));

@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -646,11 +647,13 @@ class World {
   DevSdf* h_pinned_sdfs_ = nullptr;
   DevCloth* h_pinned_cloth_ = nullptr;
   bool prims_dirty_ = true;
-  float4* stage_pos_ = nullptr;  // gather buffer of read_positions
+  std::mutex read_mutex_;        // the staging buffers and the reads out of them: threads may read one world at once
+  float4* stage_pos_ = nullptr;  // gather buffer of read_positions and of readback's fields
   float4* stage_pos2_ = nullptr;  // the second one of read_positions_async
   cudaStream_t read_stream_ = nullptr;  // copies of read_positions_async (made on first use)
   cudaEvent_t ev_gathered_[2] = {nullptr, nullptr}, ev_read_[2] = {nullptr, nullptr};
   bool read_pending_[2] = {false, false};
+  pf_status wait_staged();  // wait_reads, with read_mutex_ held
   uint32_t read_next_ = 0;
   uint64_t* prefix_dev_ = nullptr;
   uint64_t launches_per_step_ = 0;
