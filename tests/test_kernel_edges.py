@@ -580,3 +580,30 @@ def test_threads_read_one_scene_at_once(pfsim):
     with ThreadPoolExecutor(len(reads)) as pool:
         assert list(pool.map(reader, range(len(reads)))) == [0] * len(reads)
     w.close()
+
+
+def test_read_from_a_thread_on_another_device(pfsim):
+    """A thread whose current device is not the scene's reads the scene."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    import torch
+
+    from pfsim import _native as N
+    from pfsim import recipe as R
+    from pfsim import workloads as W
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    s = R.NativeBackend().build(W.dam_break(5000, seed=52))
+    s.step(1 / 60)
+    fields = [N.PF_FIELD_POSITIONS, N.PF_FIELD_DENSITY]
+
+    def elsewhere():
+        torch.cuda.set_device(1)
+        return [s.readback(f) for f in fields]
+
+    with ThreadPoolExecutor(1) as pool:
+        got = pool.submit(elsewhere).result()
+    for f, a in zip(fields, got):
+        assert np.array_equal(a, s.readback(f))
+    s.close()

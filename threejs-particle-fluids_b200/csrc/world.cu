@@ -2215,6 +2215,7 @@ pf_status World::build(const std::vector<SceneSpec*>& specs, bool use_graph, boo
   bytes_ = probe.off + al256(sort_bytes);
   if (plan_only) return PF_OK;
   (void)sm_count();  // cache the SM count outside any stream capture
+  PF_CUDA(cudaGetDevice(&device_));
   PF_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   if (const cudaError_t e = dev_alloc(&arena_, bytes_, stream_); e != cudaSuccess) {
     arena_ = nullptr;
@@ -3548,6 +3549,26 @@ pf_status World::write(uint32_t scene, uint32_t field, const void* src, size_t b
   }
 }
 
+namespace {
+// The thread's current device for its lifetime: a read launches a kernel, and
+// a thread that only reads may be on another device than the world.
+class OnDevice {
+ public:
+  explicit OnDevice(int dev) {
+    if (cudaGetDevice(&was_) == cudaSuccess && was_ != dev) moved_ = cudaSetDevice(dev) == cudaSuccess;
+  }
+  ~OnDevice() {
+    if (moved_) cudaSetDevice(was_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+
+ private:
+  int was_ = 0;
+  bool moved_ = false;
+};
+}  // namespace
+
 pf_status World::readback(uint32_t scene, uint32_t field, void* dst, size_t bytes) {
   if (scene >= specs_.size()) return fail(PF_ERR_INVALID, "readback: no such scene");
   PF_CUDA(cudaStreamSynchronize(stream_));
@@ -3571,6 +3592,7 @@ pf_status World::readback(uint32_t scene, uint32_t field, void* dst, size_t byte
   auto rows = [&](const float4* src) -> pf_status {
     PF_TRY(need(16ull * cap));
     std::lock_guard<std::mutex> lock(read_mutex_);
+    OnDevice here(device_);
     PF_TRY(wait_staged());  // an async read may still copy out of stage_pos_
     launch_slots(k_gather_rows, cap, stream_, inv, cap, src, stage_pos_);
     return fetch(16ull * cap);
@@ -3578,6 +3600,7 @@ pf_status World::readback(uint32_t scene, uint32_t field, void* dst, size_t byte
   auto words = [&](const void* src, uint32_t width, uint32_t word, bool fluid_only) -> pf_status {
     PF_TRY(need(4ull * cap));
     std::lock_guard<std::mutex> lock(read_mutex_);
+    OnDevice here(device_);
     PF_TRY(wait_staged());
     launch_slots(k_gather_words, cap, stream_, inv, cap, static_cast<const float*>(src), width, word,
                  fluid_only ? (const uint32_t*)B.tag : nullptr, reinterpret_cast<float*>(stage_pos_));

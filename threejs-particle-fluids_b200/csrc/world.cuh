@@ -614,6 +614,7 @@ class World {
   static constexpr int kSlotNbr = 0, kSlotLambda = 1, kSlotDelta = 2, kSlotVel = 3;
   Tuning tune_{};
   bool tuned_ = false;
+  int device_ = 0;  // of the stream and all memory
   // graph
   bool use_graph_ = false;
   // A plain scene's steps become a CUDA graph once it has taken kGraphAfter
